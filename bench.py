@@ -39,9 +39,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "ATV max-flow solves/s batched+served vs plain at equal Dice; p50/p99 latency"
-P_BYTES = 44   # flow sweep: tmp 4 + quat 12 + alpha 4 + hp 12 read, hp 12 written
-U_BYTES = 40   # label sweep: hp 12 + cs 4 + ct 4 + pt 4 + u 4 read, pt 4 + u 4 + tmp 4 written
-F_BYTES = 84   # one iteration (flow + labels), the algorithmic bytes per voxel-iteration
+# a sweep of two iterations: hp 12 + tmp 4 + u 4 + pt 4 + direction 12 + alpha 4 +
+# cs 4 + ct 4 read, hp 12 + tmp 4 + u 4 + pt 4 written
+PAIR_BYTES = 72
 
 
 def _rank_info():
@@ -141,7 +141,7 @@ def _peaks():
 
 
 def _traffic_summary():
-    """Per-launch DRAM bytes of the flow/label kernels from the committed ncu
+    """Per-launch DRAM bytes of the sweep kernels from the committed ncu
     summary (profiles/maxflow_traffic.json), if present."""
     path = os.path.join(ROOT, "profiles", "maxflow_traffic.json")
     try:
@@ -317,14 +317,13 @@ def run_ours(args, cfg):
     if dist:
         dist.barrier()
     ms = ev0.elapsed_time(ev1)
-    # the same solves again with every flow / label launch bracketed by CUDA
-    # events on the solve's stream: the per-kernel times of the roofline
-    p_ms = u_ms = 0.0
-    p_n = u_n = 0
+    # the same solves again with every launch of two iterations bracketed by
+    # CUDA events on the solve's stream: the kernel's time for the roofline
+    pair_ms, pair_n = 0.0, 0
     for _ in range(args.steps):
         s = N.SolveStats(1, 0, 0, 0, 0.0, 0.0, N.PATH_DEFAULT, 0)
         solve(s)
-        p_ms += s.p_ms; u_ms += s.u_ms; p_n += s.p_launches; u_n += s.u_launches
+        pair_ms += s.pair_ms; pair_n += s.pair_launches
     torch.cuda.synchronize()
     clocks = sampler.stop() if sampler else None
     if dist:
@@ -366,34 +365,26 @@ def run_ours(args, cfg):
             dist.destroy_process_group()
         return
     peak, peak_kind = _peaks()
-    p_avg = p_ms / max(p_n, 1)
-    u_avg = u_ms / max(u_n, 1)
-    p_gbs = P_BYTES * n / (p_avg * 1e-3) / 1e9
-    u_gbs = U_BYTES * n / (u_avg * 1e-3) / 1e9
+    pair_avg = pair_ms / max(pair_n, 1)
+    pair_gbs = PAIR_BYTES * n / (pair_avg * 1e-3) / 1e9
     traffic = _traffic_summary()
     tr = None
     if traffic:
-        ent = traffic.get("mf_update_p")
+        ent = traffic.get("mf_tile")
         if ent and ent.get("voxels"):
             tr = float(ent["dram_bytes_per_launch"]) * n / float(ent["voxels"])
-    # the dominant kernel of the default (two-sweep) iteration is the flow sweep
-    roof = {"bound": "hbm", "kernel": "mf_update_p_kernel (flow sweep of one max-flow iteration)",
-            "achieved": p_gbs, "peak": peak, "unit": "GB/s", "frac": p_gbs / peak, "peak_kind": peak_kind,
-            "traffic": tr, "algorithmic_bytes_per_launch": P_BYTES * n, "avg_launch_ms": p_avg}
-    it_ms = p_avg + u_avg
-    kernels = {"mf_update_p": {"avg_ms": p_avg, "launches": p_n, "GB/s": p_gbs, "frac": p_gbs / peak,
-                               "bytes_per_voxel": P_BYTES},
-               "mf_update_u": {"avg_ms": u_avg, "launches": u_n, "GB/s": u_gbs, "frac": u_gbs / peak,
-                               "bytes_per_voxel": U_BYTES},
-               "iteration": {"ms": it_ms, "GB/s": F_BYTES * n / (it_ms * 1e-3) / 1e9,
-                             "frac": F_BYTES * n / (it_ms * 1e-3) / 1e9 / peak, "bytes_per_voxel": F_BYTES,
-                             "note": "events around every launch (no launch overlap)"},
+    roof = {"bound": "hbm", "kernel": "mf_tile_kernel (two max-flow iterations per launch)",
+            "achieved": pair_gbs, "peak": peak, "unit": "GB/s", "frac": pair_gbs / peak, "peak_kind": peak_kind,
+            "traffic": tr, "algorithmic_bytes_per_launch": PAIR_BYTES * n, "avg_launch_ms": pair_avg}
+    it_ms = ms_per_step / cfg["num_iter"]
+    it_gbs = PAIR_BYTES / 2 * n / (it_ms * 1e-3) / 1e9
+    kernels = {"mf_tile": {"avg_ms": pair_avg, "launches": pair_n, "GB/s": pair_gbs, "frac": pair_gbs / peak,
+                           "bytes_per_voxel": PAIR_BYTES, "iterations_per_launch": 2,
+                           "note": "events around every launch (no launch overlap)"},
                # the timed solves themselves: launches overlap through
                # programmatic dependent launch, no events in between
-               "iteration_in_solve": {"ms": ms_per_step / cfg["num_iter"],
-                                      "GB/s": F_BYTES * n / (ms_per_step / cfg["num_iter"] * 1e-3) / 1e9,
-                                      "frac": F_BYTES * n / (ms_per_step / cfg["num_iter"] * 1e-3) / 1e9 / peak,
-                                      "bytes_per_voxel": F_BYTES}}
+               "iteration_in_solve": {"ms": it_ms, "GB/s": it_gbs, "frac": it_gbs / peak,
+                                      "bytes_per_voxel": PAIR_BYTES / 2}}
     cpu_v, kind, cpu_dt, sample = cpu_baseline(cfg, inp, iters=args.cpu_iters) if rank == 0 else (
         None, None, None, None)
     line = {"metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
@@ -913,7 +904,7 @@ def run_paths(args, cfg):
     sq = (ctypes.c_double * 3)(*np.sqrt(P.ATV_EIGS).tolist())
     stream = torch.cuda.current_stream()
 
-    def solve(timing=0, flags=0, path=N.PATH_TWO_SWEEPS):
+    def solve(timing=0, flags=0, path=N.PATH_DEFAULT):
         s = N.SolveStats(timing, 0, 0, 0, 0.0, 0.0, path, flags)
         it = ctypes.c_int32(0)
         st = L.m16_maxflow_solve_ex(N.ptr(d["img"]), N.ptr(d["quats"]), sq, None, N.ptr(d["alpha"]), 0.0,
@@ -923,7 +914,7 @@ def run_paths(args, cfg):
         N.check("m16_maxflow_solve_ex", st)
         return s
 
-    def timed(flags=0, path=N.PATH_TWO_SWEEPS):
+    def timed(flags=0, path=N.PATH_DEFAULT):
         for _ in range(args.warmup):
             solve(flags=flags, path=path)
         torch.cuda.synchronize()
@@ -935,12 +926,15 @@ def run_paths(args, cfg):
         torch.cuda.synchronize()
         k = solve(timing=1, flags=flags, path=path)
         return dict(ms_per_solve=e0.elapsed_time(e1) / args.steps, launches=s.launches,
-                    flow_sweep_ms=k.p_ms / max(k.p_launches, 1), label_sweep_ms=k.u_ms / max(k.u_launches, 1))
+                    flow_sweep_ms=k.p_ms / max(k.p_launches, 1), label_sweep_ms=k.u_ms / max(k.u_launches, 1),
+                    pair_ms=k.pair_ms / max(k.pair_launches, 1))
 
-    out = {"two_sweeps": timed()}
+    out = {"pairs": timed()}
     u_ref = u.clone()
-    out["two_sweeps_no_pdl"] = timed(flags=N.SOLVE_NO_PDL)
-    out["two_sweeps_no_pdl"]["max_u_diff_vs_pdl"] = float((u - u_ref).abs().max())
+    out["pairs_no_pdl"] = timed(flags=N.SOLVE_NO_PDL)
+    out["pairs_no_pdl"]["max_u_diff_vs_pdl"] = float((u - u_ref).abs().max())
+    out["two_sweeps"] = timed(path=N.PATH_TWO_SWEEPS)
+    out["two_sweeps"]["max_u_diff_vs_pairs"] = float((u - u_ref).abs().max())
     print(json.dumps({"workload": "launches of one %s solve, %d iterations" % ("x".join(map(str, shape)),
                                                                                 cfg["num_iter"]),
                       "steps": args.steps, "warmup": args.warmup, "paths": out}))

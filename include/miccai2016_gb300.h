@@ -56,7 +56,13 @@ typedef struct m16_cut_params {
     double scaling[3];  /* voxel size [mm/voxel] per axis, the `scaling` argument */
 } m16_cut_params;
 
-/* Workspace bytes m16_maxflow_solve needs for a (d0, d1, d2) volume. */
+/* Workspace bytes of m16_maxflow_solve for a (d0, d1, d2) volume: about 72 per
+ * voxel, for the tile sweeps (two iterations per pass over memory).  They run
+ * where the constant eigenvalues have an axis of symmetry (two of them equal).
+ * m16_maxflow_workspace_bytes_min is the least the solve accepts: about 36 per
+ * voxel, with which every iteration is a flow and a label launch, as it is for
+ * other eigenvalues and for volumes of more than 2^31 padded voxels. */
+size_t m16_maxflow_workspace_bytes_min(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 
 /*
@@ -91,11 +97,10 @@ int m16_maxflow_solve(const float *img, const float *quat3, const double *sqeval
                       float *u, int32_t *iterations, double *residuals, int32_t residuals_cap,
                       int32_t *n_residuals, void *workspace, size_t workspace_bytes, void *stream);
 
-/* Iteration paths of the single solve: a flow launch, then a label launch
- * per iteration (DEFAULT and TWO_SWEEPS are the same path).  The values 2
- * and 3 (one launch per iteration; two iterations per launch) were measured
- * slower than the two sweeps at every volume size on sm_103a and were
- * removed: they return M16_ERR_BAD_ARG. */
+/* Iteration paths of the single solve: DEFAULT runs two iterations per launch
+ * where it can (m16_maxflow_workspace_bytes), TWO_SWEEPS always a flow launch,
+ * then a label launch per iteration.  The values 2 and 3 of ABI versions 3 and
+ * 4 return M16_ERR_BAD_ARG. */
 #define M16_PATH_DEFAULT 0
 #define M16_PATH_TWO_SWEEPS 1
 
@@ -103,8 +108,8 @@ int m16_maxflow_solve(const float *img, const float *quat3, const double *sqeval
 typedef struct m16_solve_stats {
     int32_t time_kernels;  /* in: 1 brackets every flow/label kernel launch with CUDA events */
     int32_t launches;      /* out: kernels the call launched */
-    int32_t p_launches;    /* out: flow (P) kernel launches that ran */
-    int32_t u_launches;    /* out: label (U) kernel launches that ran */
+    int32_t p_launches;    /* out: flow (P) kernel launches that ran (0 with the tile sweeps) */
+    int32_t u_launches;    /* out: label (U) kernel launches that ran (0 with the tile sweeps) */
     double p_ms;           /* out: summed device time of the P launches (time_kernels only) */
     double u_ms;           /* out: summed device time of the U launches (time_kernels only) */
     int32_t path;          /* in: M16_PATH_* -- how an iteration is launched */
@@ -112,9 +117,9 @@ typedef struct m16_solve_stats {
     int32_t blocks_per_sm; /* out (m16_batch_solve): the sweeps' tile shape in use at the end, as the
                               target blocks per SM its z-chunk was chosen for; in, with
                               M16_BATCH_NO_TUNE: 8, 16 or 32 fixes that shape (0: the default) */
-    int32_t pair_launches; /* reserved (0): kept for the layout of ABI versions 3 and 4 */
-    double pair_ms;        /* reserved (0) */
-    int32_t pair_zc;       /* reserved (0) */
+    int32_t pair_launches; /* out (single solve): launches of two iterations that ran */
+    double pair_ms;        /* out (single solve): their summed device time (time_kernels only) */
+    int32_t pair_zc;       /* out (single solve): planes per block of those launches */
     int32_t reserved;
 } m16_solve_stats;
 
@@ -149,7 +154,7 @@ int m16_maxflow_solve_ex(const float *img, const float *quat3, const double *sqe
  * device memory and gives it no allocator, a foreign-language binding that
  * needs a fixed footprint known at load time, a service that must not
  * allocate while serving.  This entry point takes inputs and outputs like
- * m16_maxflow_solve but no workspace: its scratch is a fixed 11 MiB array
+ * m16_maxflow_solve but no workspace: its scratch is a fixed 22 MiB array
  * inside the library that every GPU loading the library reserves until the
  * process exits.  Nothing is allocated by the call (no cudaMalloc, no
  * allocating library routine).

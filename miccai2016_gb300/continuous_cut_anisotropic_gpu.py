@@ -53,7 +53,7 @@ class CmfCutQAnisotropicGpu(TreePrintable):
         self.last_iterations = None
         self.last_residuals = None
         self._ws = None
-        # how an iteration is launched (N.PATH_DEFAULT = N.PATH_TWO_SWEEPS)
+        # N.PATH_DEFAULT, or N.PATH_TWO_SWEEPS: a flow and a label launch per iteration
         self.iteration_path = N.PATH_DEFAULT
         self.last_stats = None
 
@@ -122,7 +122,13 @@ class CmfCutQAnisotropicGpu(TreePrintable):
                          (ctypes.c_double * 3)(*scaling))
         nbytes = L.m16_maxflow_workspace_bytes(shape[0], shape[1], shape[2], ctypes.byref(cp))
         if self._ws is None or self._ws.numel() < nbytes:
-            self._ws = N.workspace(nbytes)
+            self._ws = None
+            try:
+                self._ws = N.workspace(nbytes)
+            except torch.cuda.OutOfMemoryError:
+                # the smaller workspace of the two sweeps
+                self._ws = N.workspace(L.m16_maxflow_workspace_bytes_min(shape[0], shape[1], shape[2],
+                                                                         ctypes.byref(cp)))
         cap = int(p.num_iter) // max(int(p.update), 1) + 2
         resid = (ctypes.c_double * cap)()
         iters = ctypes.c_int32(0)

@@ -4,15 +4,18 @@
 // in CmfCutQAnisotropicGpu._execute
 // (src/processing/continuous_cut_anisotropic_gpu.py:198-344).
 //
-// Data layout in HBM (one solve, N voxels, all fp32, C order z-y-x):
-//   caller:    img, quat3 (N x 3), alpha (N or scalar), cs, ct, labels (u8), u (output/state)
-//   workspace: hp0, hp1, hp2, pt, tmp (N each), q4 (N x float4, the expanded
-//              quaternion), block partials, control word, residual log.
-//
-// Per iteration two kernels run:
+// A solve whose constant eigenvalues have an axis of symmetry (two of them
+// equal: the anisotropic and the isotropic cut) runs two iterations per pass
+// over memory (maxflow_tile.cuh, tile_sweep.cuh).  Other eigenvalues, per-voxel
+// ones, volumes beyond 32-bit indexes and callers with a small workspace take
+// two sweeps per iteration:
 //   P: hp <- project_alpha(H^-1 hp + steps * H^T grad(tmp)), hp <- H p
 //   U: div(hp), p_s, p_t, u and tmp = err - u / cc (update_tmp fused), and on
 //      check iterations the |err| partial sums of the residual.
+// Data layout in HBM of the two sweeps (N voxels, all fp32, C order z-y-x):
+//   caller:    img, quat3 (N x 3), alpha (N or scalar), cs, ct, labels (u8), u (output/state)
+//   workspace: hp0, hp1, hp2, pt, tmp (N each), q4 (N x float4, the expanded
+//              quaternion), block partials, control word, residual log.
 // Each thread marches along z through a column of the volume; x/y neighbours
 // come from L1, the z neighbour is carried in a register.  The quaternion is
 // expanded once per solve so the iterations need no trigonometry.
@@ -35,7 +38,7 @@ struct MfCtrl {
     int stopped;      // 1 once a check stopped the solve
     int iterations;   // iterations executed
     int n_checks;     // residual checks done
-    int pad0;
+    int error;        // a copy of the tile sweeps did not arrive in time
     float denom;      // max(img) + FLT_MIN
     float pad1[3];
 };
@@ -94,6 +97,7 @@ __global__ void mf_init_ctrl_kernel(const float *__restrict__ part, int nparts, 
     ctrl->stopped = 0;
     ctrl->iterations = num_iter;
     ctrl->n_checks = 0;
+    ctrl->error = 0;
 }
 
 // hp = 0, p_t = fmin(cs, ct), u = img / denom, tmp = -u * rcc, q4 = qexpand(quat3)
@@ -256,12 +260,21 @@ inline bool finite_pos(double v) { return v > 0.0 && v < 1e300; }
 }  // namespace
 }  // namespace m16
 
+#include "maxflow_tile.cuh"
+
 using namespace m16;
 
-extern "C" size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
+extern "C" size_t m16_maxflow_workspace_bytes_min(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
 {
     if (d0 < 1 || d1 < 1 || d2 < 1 || !params) return 0;
     return mf_layout(d0, d1, d2, params->num_iter, params->update).total;
+}
+
+extern "C" size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
+{
+    const size_t two_sweeps = m16_maxflow_workspace_bytes_min(d0, d1, d2, params);
+    if (!two_sweeps || !tile_shape_ok(d0, d1, d2)) return two_sweeps;
+    return std::max(two_sweeps, mf_tile_layout(d0, d1, d2, params->num_iter, params->update).total);
 }
 
 extern "C" int m16_maxflow_solve(const float *img, const float *quat3, const double *sqevals3,
@@ -295,7 +308,163 @@ struct EventPool {
 };
 }  // namespace
 
-// The solve: every iteration a flow and a label launch.
+namespace {
+
+// The solve over the tile sweeps (maxflow_tile.cuh), `axis` and V's metric
+// from tile_metric; the arguments have been checked.
+int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView V, const float *alpha,
+                        float alpha_scalar, const float *cs, const float *ct, const uint8_t *labels, int d0, int d1,
+                        int d2, const m16_cut_params *params, float *u, int32_t *iterations, double *residuals,
+                        int32_t residuals_cap, int32_t *n_residuals, const MfTileLayout &L, char *ws, cudaStream_t st,
+                        m16_solve_stats *stats)
+{
+    const int64_t n = (int64_t)d0 * d1 * d2;
+    const bool dir = axis < 3, array = alpha != nullptr;
+    const double *sc = params->scaling;
+    const double smin = fmin(sc[0], fmin(sc[1], sc[2]));
+    const double rcc = 1.0 / (params->cc * (smin * smin));
+    MfCtrl *ctrl = (MfCtrl *)(ws + L.ctrl);
+    double *resid = (double *)(ws + L.resid);
+    V.d0 = d0; V.d1 = d1; V.d2 = d2; V.pitch = tile_pitch(d2);
+    V.ss0 = (float)(params->steps / sc[0] * (smin * smin));
+    V.ss1 = (float)(params->steps / sc[1] * (smin * smin));
+    V.ss2 = (float)(params->steps / sc[2] * (smin * smin));
+    V.rs0 = (float)(1.0 / sc[0]); V.rs1 = (float)(1.0 / sc[1]); V.rs2 = (float)(1.0 / sc[2]);
+    V.rcc = (float)rcc;
+    V.ircc = (float)(1.0 / rcc);
+    V.alpha_scalar = alpha_scalar;
+    V.w = 0.f; V.nid2 = 0.f;
+    V.labels = labels;
+    V.err = &ctrl->error;
+    // the two directions of a sweep: buffer k read, the other written
+    MfTileArgs args[2];
+    for (int k = 0; k < 2; ++k) {
+        MfTileArgs &a = args[k];
+        a.V = V;
+        a.V.ho = (float4 *)(ws + L.h[1 - k]);
+        a.V.uo = (float2 *)(ws + L.u[1 - k]);
+        a.nx = L.nx; a.ny = L.ny; a.zc = L.zc;
+        a.partials = (float *)(ws + L.partials);
+        a.stopped = &ctrl->stopped;
+        bool ok = tile_map(&a.mh, ws + L.h[k], d0, d1, V.pitch, 4, kTileRows + 1) &&
+                  tile_map(&a.mu, ws + L.u[k], d0, d1, V.pitch, 2, kTileRows) &&
+                  tile_map(&a.mcaps, ws + L.caps, d0, d1, V.pitch, 2, kTileRows);
+        ok = ok && tile_map(&a.mdir, ws + L.dir, d0, d1, V.pitch, 4, kTileRows);
+        ok = ok && tile_map(&a.mrad, ws + L.dir, d0, d1, V.pitch, 1, kTileRows);   // in place of the directions
+        if (!ok) return M16_ERR_CUDA;
+    }
+    MfTileLaunch kernels[2][2];   // [iterations - 1][check]
+    for (int k = 0; k < 2; ++k)
+        for (int c = 0; c < 2; ++c) {
+            kernels[k][c] = mf_tile_pick(dir, array, labels != nullptr, k + 1, c != 0);
+            M16_CUDA_TRY(cudaFuncSetAttribute(kernels[k][c].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kernels[k][c].smem));
+        }
+
+    const int init_blocks = (int)std::min<int64_t>(kMaxBlocks, div_up(n, 256));
+    mf_max_kernel<<<init_blocks, 256, 0, st>>>(img, n, (float *)(ws + L.maxpart));
+    mf_init_ctrl_kernel<<<1, 32, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, ctrl);
+    mf_tile_init_kernel<<<init_blocks, 256, 0, st>>>(
+        img, quat3, alpha, alpha_scalar, cs, ct, d2, (int64_t)d0 * d1, V.rcc, axis % 3, ctrl, (float4 *)(ws + L.h[0]),
+        (float2 *)(ws + L.u[0]), (float2 *)(ws + L.caps), dir ? (float4 *)(ws + L.dir) : nullptr,
+        !dir && array ? (float *)(ws + L.dir) : nullptr);
+    M16_CUDA_TRY(cudaGetLastError());
+    int launches = 3;
+
+    const int num_iter = params->num_iter, update = params->update;
+    // iterations between two looks at the stopping state: even, so that pairs
+    // start at even iterations; without a bound only a NaN residual stops
+    int chunk = update * std::max(1, 64 / update);
+    chunk += chunk & 1;
+    if (!(params->error_bound > 0.0)) chunk = std::max(chunk, 1024);
+    const bool timing = stats && stats->time_kernels;
+    const bool pdl = !(stats && (stats->flags & M16_SOLVE_NO_PDL));
+    std::unique_ptr<EventPool> pool;
+    if (timing) {
+        pool.reset(new EventPool(std::min(num_iter, chunk) + 2));
+        if (!pool->ok) return M16_ERR_CUDA;
+    }
+    auto sweep = [&](int count, bool check, int buf, bool always) -> cudaError_t {
+        const MfTileLaunch &K = kernels[count - 1][check];
+        MfTileArgs a = args[buf];
+        if (always) a.stopped = nullptr;
+        return launch_pdl_smem(K.kernel, dim3(L.nblocks), dim3(kTileLanes, kTileNW), K.smem, st, pdl, a);
+    };
+    int pair_n = 0;
+    double pair_ms = 0.0;
+    MfCtrl hctrl;
+    hctrl.stopped = 0;
+    int it = 0;
+    while (it < num_iter) {
+        const int end = std::min(num_iter, it + chunk), begin = it;
+        int slots = 0;
+        while (it < end) {
+            const int count = std::min(2, num_iter - it);
+            const bool check = it % update == 0 || (count == 2 && (it + 1) % update == 0);
+            const bool time_it = timing && count == 2;
+            if (time_it) cudaEventRecord(pool->ev[2 * slots], st);
+            M16_CUDA_TRY(sweep(count, check, (it >> 1) & 1, false));
+            if (time_it) cudaEventRecord(pool->ev[2 * slots++ + 1], st);
+            ++launches;
+            if (check) {
+                M16_CUDA_TRY(launch_pdl(mf_tile_check_kernel, dim3(1), dim3(256), st, pdl,
+                                        (const float *)(ws + L.partials), L.nblocks, 1.0 / ((double)n * rcc),
+                                        params->error_bound, it, count, update, L.resid_cap, ctrl, resid));
+                ++launches;
+            }
+            it += count;
+        }
+        M16_CUDA_TRY(cudaGetLastError());
+        M16_CUDA_TRY(cudaMemcpyAsync(&hctrl, ctrl, sizeof(MfCtrl), cudaMemcpyDeviceToHost, st));
+        M16_CUDA_TRY(cudaStreamSynchronize(st));
+        for (int j = 0; j < slots; ++j) {
+            // only pairs that ran (not the no-op launches after a stop) count
+            if (hctrl.stopped && begin + 2 * j >= hctrl.iterations) break;
+            float ms = 0.f;
+            M16_CUDA_TRY(cudaEventElapsedTime(&ms, pool->ev[2 * j], pool->ev[2 * j + 1]));
+            pair_ms += ms;
+            ++pair_n;
+        }
+        if (hctrl.stopped) break;
+    }
+    if (num_iter == 0) {
+        M16_CUDA_TRY(cudaMemcpyAsync(&hctrl, ctrl, sizeof(MfCtrl), cudaMemcpyDeviceToHost, st));
+        M16_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    if (hctrl.error) return M16_ERR_TIMEOUT;
+    const int ran = hctrl.stopped ? hctrl.iterations : it;
+    // stopped by the check of a pair's first iteration: that one again, alone,
+    // from the buffer the pair read
+    if (ran & 1 && ran < num_iter) {
+        M16_CUDA_TRY(sweep(1, false, (ran >> 1) & 1, true));
+        ++launches;
+    }
+    mf_tile_result_kernel<<<init_blocks, 256, 0, st>>>((const float2 *)(ws + L.u[((ran + 1) >> 1) & 1]), d2, n, u);
+    ++launches;
+    M16_CUDA_TRY(cudaGetLastError());
+    if (stats) {
+        stats->launches = launches;
+        stats->p_launches = stats->u_launches = 0;   // no separate flow and label launches
+        stats->p_ms = stats->u_ms = 0.0;
+        stats->pair_launches = timing ? pair_n : ran / 2;
+        stats->pair_ms = pair_ms;
+        stats->pair_zc = L.zc;
+    }
+    *iterations = hctrl.iterations;
+    if (n_residuals) *n_residuals = hctrl.n_checks;
+    if (residuals && residuals_cap > 0) {
+        const int cnt = std::min(std::min(hctrl.n_checks, residuals_cap), L.resid_cap);
+        if (cnt > 0) M16_CUDA_TRY(cudaMemcpyAsync(residuals, resid, (size_t)cnt * 8, cudaMemcpyDeviceToHost, st));
+    }
+    M16_CUDA_TRY(cudaStreamSynchronize(st));
+    return M16_OK;
+}
+
+}  // namespace
+
+// The solve: over the tile sweeps where the constant eigenvalues have an axis
+// of symmetry and the workspace holds their fields, else every iteration a
+// flow and a label launch.
 static int maxflow_solve_impl(const float *img, const float *quat3, const double *sqevals3, const float *sqeigs,
                               const float *alpha, float alpha_scalar, const float *cs, const float *ct,
                               const uint8_t *labels, int32_t d0, int32_t d1, int32_t d2,
@@ -319,6 +488,17 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
     cudaStream_t st = (cudaStream_t)stream;
     char *ws = (char *)workspace;
     const int64_t n = (int64_t)d0 * d1 * d2;
+    // Two iterations a pass over 72 bytes a voxel (256^3: 95 us an iteration)
+    // against two passes an iteration over 88 (228 us); the two sweeps take half
+    // the workspace, any eigenvalues and any volume size.
+    if (sqevals3 && tile_shape_ok(d0, d1, d2) && !(stats && stats->path == M16_PATH_TWO_SWEEPS)) {
+        TileView V = TileView();
+        const int axis = tile_metric(sqevals3, V);
+        const MfTileLayout T = mf_tile_layout(d0, d1, d2, params->num_iter, params->update);
+        if (axis >= 0 && workspace_bytes >= T.total)
+            return maxflow_solve_tiles(img, quat3, axis, V, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2, params, u,
+                                       iterations, residuals, residuals_cap, n_residuals, T, ws, st, stats);
+    }
 
     // constants as _reinit_clprograms derives them (continuous_cut_anisotropic_gpu.py:104-129)
     const double *sc = params->scaling;
@@ -459,8 +639,6 @@ extern "C" int m16_maxflow_solve_ex(const float *img, const float *quat3, const 
                                     int32_t *n_residuals, void *workspace, size_t workspace_bytes, void *stream,
                                     m16_solve_stats *stats)
 {
-    // the two sweeps are the only iteration path (the fused iteration and two
-    // iterations per launch measured slower at every size and were removed)
     if (stats && stats->path != M16_PATH_DEFAULT && stats->path != M16_PATH_TWO_SWEEPS) return M16_ERR_BAD_ARG;
     return maxflow_solve_impl(img, quat3, sqevals3, sqeigs, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2, params,
                               u, iterations, residuals, residuals_cap, n_residuals, workspace, workspace_bytes,
@@ -485,10 +663,11 @@ namespace m16 {
 namespace {
 constexpr int64_t kStaticMaxVoxels = 262144;
 constexpr int kStaticMaxChecks = 4096;
-// hp0, hp1, hp2, pt, tmp (4 B each) + q4 (16 B) + block partials (<= 4 B per voxel,
-// every block covers at least one voxel) + max partials + control + residual log,
-// each region rounded up to 256 B
-constexpr size_t kStaticBytes = 11u << 20;   // 11 MiB >= 10,521,344 B needed at the limits
+// 72 B per padded voxel of the tile sweeps (at most 294,912 of them,
+// tile_shape_ok) or 36 B per voxel of the two sweeps, block partials (<= 8 B per
+// voxel, every block covers at least one voxel; the tile sweeps' far fewer),
+// max partials, control and residual log, each region rounded up to 256 B
+constexpr size_t kStaticBytes = 22u << 20;   // 22 MiB >= 21,270,000 B needed at the limits
 
 }  // namespace
 }  // namespace m16
@@ -533,7 +712,6 @@ extern "C" int m16_maxflow_solve_static(const float *img, const float *quat3, co
     // The solve's initialisation kernels write every scratch word before it is
     // read (flow state, control word, partial sums), so nothing of the previous
     // call's contents leaks into this one.
-    // the two-sweep iteration: its workspace fits the fixed array
     return maxflow_solve_impl(img, quat3, sqevals3, sqeigs, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2, params,
                               u, iterations, residuals, residuals_cap, n_residuals, scratch, kStaticBytes, stream,
                               nullptr);
