@@ -56,12 +56,11 @@ typedef struct m16_cut_params {
     double scaling[3];  /* voxel size [mm/voxel] per axis, the `scaling` argument */
 } m16_cut_params;
 
-/* Workspace bytes of m16_maxflow_solve for a (d0, d1, d2) volume: about 72 per
- * voxel, for the tile sweeps (two iterations per pass over memory).  They run
- * where the constant eigenvalues have an axis of symmetry (two of them equal).
- * m16_maxflow_workspace_bytes_min is the least the solve accepts: about 36 per
- * voxel, with which every iteration is a flow and a label launch, as it is for
- * other eigenvalues and for volumes of more than 2^31 padded voxels. */
+/* Workspace bytes of m16_maxflow_solve for a (d0, d1, d2) volume: about 88 per
+ * voxel, for the tile sweeps (two iterations per pass over memory; 76 do with
+ * constant eigenvalues).  m16_maxflow_workspace_bytes_min is the least the
+ * solve accepts: about 36 per voxel, with which every iteration is a flow and
+ * a label launch, as it is for volumes of more than 2^31 padded voxels. */
 size_t m16_maxflow_workspace_bytes_min(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 
@@ -154,7 +153,7 @@ int m16_maxflow_solve_ex(const float *img, const float *quat3, const double *sqe
  * device memory and gives it no allocator, a foreign-language binding that
  * needs a fixed footprint known at load time, a service that must not
  * allocate while serving.  This entry point takes inputs and outputs like
- * m16_maxflow_solve but no workspace: its scratch is a fixed 22 MiB array
+ * m16_maxflow_solve but no workspace: its scratch is a fixed 25 MiB array
  * inside the library that every GPU loading the library reserves until the
  * process exits.  Nothing is allocated by the call (no cudaMalloc, no
  * allocating library routine).

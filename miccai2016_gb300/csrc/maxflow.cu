@@ -4,11 +4,9 @@
 // in CmfCutQAnisotropicGpu._execute
 // (src/processing/continuous_cut_anisotropic_gpu.py:198-344).
 //
-// A solve whose constant eigenvalues have an axis of symmetry (two of them
-// equal: the anisotropic and the isotropic cut) runs two iterations per pass
-// over memory (maxflow_tile.cuh, tile_sweep.cuh).  Other eigenvalues, per-voxel
-// ones, volumes beyond 32-bit indexes and callers with a small workspace take
-// two sweeps per iteration:
+// A solve runs two iterations per pass over memory (maxflow_tile.cuh,
+// tile_sweep.cuh).  Volumes beyond 32-bit indexes and callers with a small
+// workspace take two sweeps per iteration:
 //   P: hp <- project_alpha(H^-1 hp + steps * H^T grad(tmp)), hp <- H p
 //   U: div(hp), p_s, p_t, u and tmp = err - u / cc (update_tmp fused), and on
 //      check iterations the |err| partial sums of the residual.
@@ -274,7 +272,7 @@ extern "C" size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2
 {
     const size_t two_sweeps = m16_maxflow_workspace_bytes_min(d0, d1, d2, params);
     if (!two_sweeps || !tile_shape_ok(d0, d1, d2)) return two_sweeps;
-    return std::max(two_sweeps, mf_tile_layout(d0, d1, d2, params->num_iter, params->update).total);
+    return std::max(two_sweeps, mf_tile_layout(d0, d1, d2, params->num_iter, params->update, true).total);
 }
 
 extern "C" int m16_maxflow_solve(const float *img, const float *quat3, const double *sqevals3,
@@ -310,16 +308,18 @@ struct EventPool {
 
 namespace {
 
-// The solve over the tile sweeps (maxflow_tile.cuh), `axis` and V's metric
-// from tile_metric; the arguments have been checked.
-int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView V, const float *alpha,
-                        float alpha_scalar, const float *cs, const float *ct, const uint8_t *labels, int d0, int d1,
-                        int d2, const m16_cut_params *params, float *u, int32_t *iterations, double *residuals,
-                        int32_t residuals_cap, int32_t *n_residuals, const MfTileLayout &L, char *ws, cudaStream_t st,
-                        m16_solve_stats *stats)
+// The solve over the tile sweeps (maxflow_tile.cuh); the arguments have been
+// checked.
+int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqevals3, const float *sqeigs,
+                        const float *alpha, float alpha_scalar, const float *cs, const float *ct,
+                        const uint8_t *labels, int d0, int d1, int d2, const m16_cut_params *params, float *u,
+                        int32_t *iterations, double *residuals, int32_t residuals_cap, int32_t *n_residuals,
+                        const MfTileLayout &L, char *ws, cudaStream_t st, m16_solve_stats *stats)
 {
     const int64_t n = (int64_t)d0 * d1 * d2;
-    const bool dir = axis < 3, array = alpha != nullptr;
+    TileView V = TileView();
+    int axis = -1;
+    const int metric = sqevals3 ? tile_metric(sqevals3, V, &axis) : kMetricField;
     const double *sc = params->scaling;
     const double smin = fmin(sc[0], fmin(sc[1], sc[2]));
     const double rcc = 1.0 / (params->cc * (smin * smin));
@@ -332,8 +332,6 @@ int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView
     V.rs0 = (float)(1.0 / sc[0]); V.rs1 = (float)(1.0 / sc[1]); V.rs2 = (float)(1.0 / sc[2]);
     V.rcc = (float)rcc;
     V.ircc = (float)(1.0 / rcc);
-    V.alpha_scalar = alpha_scalar;
-    V.w = 0.f; V.nid2 = 0.f;
     V.labels = labels;
     V.err = &ctrl->error;
     // the two directions of a sweep: buffer k read, the other written
@@ -349,14 +347,15 @@ int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView
         bool ok = tile_map(&a.mh, ws + L.h[k], d0, d1, V.pitch, 4, kTileRows + 1) &&
                   tile_map(&a.mu, ws + L.u[k], d0, d1, V.pitch, 2, kTileRows) &&
                   tile_map(&a.mcaps, ws + L.caps, d0, d1, V.pitch, 2, kTileRows);
-        ok = ok && tile_map(&a.mdir, ws + L.dir, d0, d1, V.pitch, 4, kTileRows);
-        ok = ok && tile_map(&a.mrad, ws + L.dir, d0, d1, V.pitch, 1, kTileRows);   // in place of the directions
+        if (metric != kMetricIso) ok = ok && tile_map(&a.mdir, ws + L.dir, d0, d1, V.pitch, 4, kTileRows);
+        if (metric == kMetricField) ok = ok && tile_map(&a.meig, ws + L.eig, d0, d1, V.pitch, 4, kTileRows);
+        else ok = ok && tile_map(&a.mrad, ws + L.eig, d0, d1, V.pitch, 1, kTileRows);
         if (!ok) return M16_ERR_CUDA;
     }
     MfTileLaunch kernels[2][2];   // [iterations - 1][check]
     for (int k = 0; k < 2; ++k)
         for (int c = 0; c < 2; ++c) {
-            kernels[k][c] = mf_tile_pick(dir, array, labels != nullptr, k + 1, c != 0);
+            kernels[k][c] = labels ? mf_tile_pick<true>(metric, k + 1, c != 0) : mf_tile_pick<false>(metric, k + 1, c != 0);
             M16_CUDA_TRY(cudaFuncSetAttribute(kernels[k][c].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kernels[k][c].smem));
         }
@@ -364,10 +363,12 @@ int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView
     const int init_blocks = (int)std::min<int64_t>(kMaxBlocks, div_up(n, 256));
     mf_max_kernel<<<init_blocks, 256, 0, st>>>(img, n, (float *)(ws + L.maxpart));
     mf_init_ctrl_kernel<<<1, 32, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, ctrl);
+    const bool planar = metric == kMetricIso || metric == kMetricConst;
     mf_tile_init_kernel<<<init_blocks, 256, 0, st>>>(
-        img, quat3, alpha, alpha_scalar, cs, ct, d2, (int64_t)d0 * d1, V.rcc, axis % 3, ctrl, (float4 *)(ws + L.h[0]),
-        (float2 *)(ws + L.u[0]), (float2 *)(ws + L.caps), dir ? (float4 *)(ws + L.dir) : nullptr,
-        !dir && array ? (float *)(ws + L.dir) : nullptr);
+        img, quat3, sqeigs, alpha, alpha_scalar, cs, ct, d2, (int64_t)d0 * d1, V.rcc, axis, ctrl,
+        (float4 *)(ws + L.h[0]), (float2 *)(ws + L.u[0]), (float2 *)(ws + L.caps),
+        metric != kMetricIso ? (float4 *)(ws + L.dir) : nullptr,
+        metric == kMetricField ? (float4 *)(ws + L.eig) : nullptr, planar ? (float *)(ws + L.eig) : nullptr);
     M16_CUDA_TRY(cudaGetLastError());
     int launches = 3;
 
@@ -462,9 +463,8 @@ int maxflow_solve_tiles(const float *img, const float *quat3, int axis, TileView
 
 }  // namespace
 
-// The solve: over the tile sweeps where the constant eigenvalues have an axis
-// of symmetry and the workspace holds their fields, else every iteration a
-// flow and a label launch.
+// The solve: over the tile sweeps where the workspace holds their fields, else
+// every iteration a flow and a label launch.
 static int maxflow_solve_impl(const float *img, const float *quat3, const double *sqevals3, const float *sqeigs,
                               const float *alpha, float alpha_scalar, const float *cs, const float *ct,
                               const uint8_t *labels, int32_t d0, int32_t d1, int32_t d2,
@@ -490,14 +490,12 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
     const int64_t n = (int64_t)d0 * d1 * d2;
     // Two iterations a pass over 72 bytes a voxel (256^3: 95 us an iteration)
     // against two passes an iteration over 88 (228 us); the two sweeps take half
-    // the workspace, any eigenvalues and any volume size.
-    if (sqevals3 && tile_shape_ok(d0, d1, d2) && !(stats && stats->path == M16_PATH_TWO_SWEEPS)) {
-        TileView V = TileView();
-        const int axis = tile_metric(sqevals3, V);
-        const MfTileLayout T = mf_tile_layout(d0, d1, d2, params->num_iter, params->update);
-        if (axis >= 0 && workspace_bytes >= T.total)
-            return maxflow_solve_tiles(img, quat3, axis, V, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2, params, u,
-                                       iterations, residuals, residuals_cap, n_residuals, T, ws, st, stats);
+    // the workspace and any volume size.
+    if (tile_shape_ok(d0, d1, d2) && !(stats && stats->path == M16_PATH_TWO_SWEEPS)) {
+        const MfTileLayout T = mf_tile_layout(d0, d1, d2, params->num_iter, params->update, sqevals3 == nullptr);
+        if (workspace_bytes >= T.total)
+            return maxflow_solve_tiles(img, quat3, sqevals3, sqeigs, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2,
+                                       params, u, iterations, residuals, residuals_cap, n_residuals, T, ws, st, stats);
     }
 
     // constants as _reinit_clprograms derives them (continuous_cut_anisotropic_gpu.py:104-129)
@@ -663,11 +661,11 @@ namespace m16 {
 namespace {
 constexpr int64_t kStaticMaxVoxels = 262144;
 constexpr int kStaticMaxChecks = 4096;
-// 72 B per padded voxel of the tile sweeps (at most 294,912 of them,
-// tile_shape_ok) or 36 B per voxel of the two sweeps, block partials (<= 8 B per
-// voxel, every block covers at least one voxel; the tile sweeps' far fewer),
-// max partials, control and residual log, each region rounded up to 256 B
-constexpr size_t kStaticBytes = 22u << 20;   // 22 MiB >= 21,270,000 B needed at the limits
+// 88 B per padded voxel of the tile sweeps (at most 294,912 of them,
+// tile_shape_ok), 8 B per block of theirs (at least 208 voxels each, or all of a
+// small volume), max partials, control and residual log, each region rounded up
+// to 256 B; the two sweeps take less than half of it
+constexpr size_t kStaticBytes = 25u << 20;   // 25 MiB >= 25,990,000 B needed at the limits
 
 }  // namespace
 }  // namespace m16

@@ -14,29 +14,29 @@ namespace m16 {
 namespace {
 
 struct MfTileArgs {
-    CUtensorMap mh, mu, mdir, mcaps, mrad;
+    CUtensorMap mh, mu, mdir, meig, mcaps, mrad;
     TileView V;
     int nx, ny, zc;
     float *partials;        // per block: iteration 0, then iteration 1
     const int *stopped;     // null: run whatever the solve's state
 };
 
-template <int K, bool DIR, int ASRC, bool SUP, bool CHECK>
+template <int K, int METRIC, int ASRC, bool SUP, bool CHECK>
 __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) mf_tile_kernel(const __grid_constant__ MfTileArgs a)
 {
     extern __shared__ __align__(128) unsigned char tile_mem[];
     __shared__ float red[32];
-    TileMem<DIR, ASRC> &M = *reinterpret_cast<TileMem<DIR, ASRC> *>(tile_mem);
+    TileMem<METRIC, ASRC> &M = *reinterpret_cast<TileMem<METRIC, ASRC> *>(tile_mem);
     tile_init(M);
     pdl_wait();
     pdl_launch_next();
     if (a.stopped && __ldcg(a.stopped)) return;
     TileView V = a.V;
-    V.mh = &a.mh; V.mu = &a.mu; V.mdir = &a.mdir; V.mcaps = &a.mcaps; V.mrad = &a.mrad;
+    V.mh = &a.mh; V.mu = &a.mu; V.mdir = &a.mdir; V.meig = &a.meig; V.mcaps = &a.mcaps; V.mrad = &a.mrad;
     const int bx = blockIdx.x % a.nx, t = blockIdx.x / a.nx;
     const int by = t % a.ny, za = t / a.ny * a.zc;
     float acc[2] = {0.f, 0.f};
-    tile_sweep<K, DIR, ASRC, false, SUP, CHECK>(V, M, bx, by, za, min(za + a.zc, V.d0), acc);
+    tile_sweep<K, METRIC, ASRC, false, SUP, CHECK>(V, M, bx, by, za, min(za + a.zc, V.d0), acc);
     if (CHECK) {
         const float s0 = block_sum(acc[0], red);
         __syncthreads();
@@ -49,13 +49,15 @@ __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) mf_tile_kern
 }
 
 // the padded fields: h4 = (0, 0, 0, -u rcc), u2 = (u, fmin(cs, ct)) with u =
-// img / denom (continuous_cut_anisotropic_gpu.py:276-289), caps, and the
-// direction (column `axis` of the rotation) with the radius or the radius alone
+// img / denom (continuous_cut_anisotropic_gpu.py:276-289), caps; where given,
+// dir (column `axis` of the rotation and the radius, or the quaternion for
+// axis < 0), eig (square roots of the eigenvalues and the radius) and rad
 __global__ void mf_tile_init_kernel(const float *__restrict__ img, const float *__restrict__ quat3,
-                                    const float *__restrict__ alpha, float alpha_scalar, const float *__restrict__ cs,
-                                    const float *__restrict__ ct, int d2, int64_t rows, float rcc, int axis,
-                                    const MfCtrl *ctrl, float4 *__restrict__ h4, float2 *__restrict__ u2,
-                                    float2 *__restrict__ caps, float4 *__restrict__ dir, float *__restrict__ rad)
+                                    const float *__restrict__ sqeigs, const float *__restrict__ alpha,
+                                    float alpha_scalar, const float *__restrict__ cs, const float *__restrict__ ct,
+                                    int d2, int64_t rows, float rcc, int axis, const MfCtrl *ctrl,
+                                    float4 *__restrict__ h4, float2 *__restrict__ u2, float2 *__restrict__ caps,
+                                    float4 *__restrict__ dir, float4 *__restrict__ eig, float *__restrict__ rad)
 {
     const float denom = ctrl->denom;
     const int pitch = tile_pitch(d2);
@@ -67,6 +69,7 @@ __global__ void mf_tile_init_kernel(const float *__restrict__ img, const float *
             h4[o] = make_float4(0.f, 0.f, 0.f, 0.f);
             u2[o] = caps[o] = make_float2(0.f, 0.f);
             if (dir) dir[o] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (eig) eig[o] = make_float4(1.f, 1.f, 1.f, 0.f);
             if (rad) rad[o] = 0.f;
             continue;
         }
@@ -76,7 +79,9 @@ __global__ void mf_tile_init_kernel(const float *__restrict__ img, const float *
         u2[o] = make_float2(u, fminf(c, t));
         caps[o] = make_float2(c, t);
         const float r = alpha ? alpha[i] : alpha_scalar;
-        if (dir) dir[o] = tile_direction(quat3 + 3 * i, axis, r);
+        if (dir) dir[o] = axis < 0 ? qexpand(quat3[3 * i], quat3[3 * i + 1], quat3[3 * i + 2])
+                                   : tile_direction(quat3 + 3 * i, axis, r);
+        if (eig) eig[o] = make_float4(sqeigs[3 * i], sqeigs[3 * i + 1], sqeigs[3 * i + 2], r);
         if (rad) rad[o] = r;
     }
 }
@@ -129,11 +134,11 @@ __global__ void mf_tile_check_kernel(const float *__restrict__ part, int nparts,
 }
 
 struct MfTileLayout {
-    size_t h[2], u[2], dir, caps, partials, maxpart, ctrl, resid, total;
+    size_t h[2], u[2], dir, eig, caps, partials, maxpart, ctrl, resid, total;
     int nx, ny, zc, nblocks, resid_cap;
 };
 
-inline MfTileLayout mf_tile_layout(int d0, int d1, int d2, int num_iter, int update)
+inline MfTileLayout mf_tile_layout(int d0, int d1, int d2, int num_iter, int update, bool field)
 {
     MfTileLayout L;
     const size_t np = (size_t)tile_voxels(d0, d1, d2);
@@ -149,6 +154,7 @@ inline MfTileLayout mf_tile_layout(int d0, int d1, int d2, int num_iter, int upd
         L.u[k] = take(np * 8);
     }
     L.dir = take(np * 16);
+    L.eig = take(np * (field ? 16 : 4));   // the eigenvalues' field, or the radius alone
     L.caps = take(np * 8);
     L.partials = take((size_t)L.nblocks * 8);
     L.maxpart = take(kMaxBlocks * 4);
@@ -165,25 +171,25 @@ struct MfTileLaunch {
     size_t smem;
 };
 
-template <bool DIR, int ASRC, bool SUP>
+template <int METRIC, int ASRC, bool SUP>
 MfTileLaunch mf_tile_kernel_of(int k, bool check)
 {
     MfTileLaunch L;
-    L.smem = sizeof(TileMem<DIR, ASRC>);
-    if (k == 2) L.kernel = check ? mf_tile_kernel<2, DIR, ASRC, SUP, true> : mf_tile_kernel<2, DIR, ASRC, SUP, false>;
-    else L.kernel = check ? mf_tile_kernel<1, DIR, ASRC, SUP, true> : mf_tile_kernel<1, DIR, ASRC, SUP, false>;
+    L.smem = sizeof(TileMem<METRIC, ASRC>);
+    if (k == 2) L.kernel = check ? mf_tile_kernel<2, METRIC, ASRC, SUP, true> : mf_tile_kernel<2, METRIC, ASRC, SUP, false>;
+    else L.kernel = check ? mf_tile_kernel<1, METRIC, ASRC, SUP, true> : mf_tile_kernel<1, METRIC, ASRC, SUP, false>;
     return L;
 }
 
-// direction (1), radius array (2), seeds (4)
-inline MfTileLaunch mf_tile_pick(bool dir, bool array, bool sup, int k, bool check)
+template <bool SUP>
+MfTileLaunch mf_tile_pick(int metric, int k, bool check)
 {
-    if (dir) return sup ? mf_tile_kernel_of<true, kRadPacked, true>(k, check)
-                        : mf_tile_kernel_of<true, kRadPacked, false>(k, check);
-    if (array) return sup ? mf_tile_kernel_of<false, kRadPlanar, true>(k, check)
-                          : mf_tile_kernel_of<false, kRadPlanar, false>(k, check);
-    return sup ? mf_tile_kernel_of<false, kRadScalar, true>(k, check)
-               : mf_tile_kernel_of<false, kRadScalar, false>(k, check);
+    switch (metric) {
+        case kMetricIso: return mf_tile_kernel_of<kMetricIso, kRadPlanar, SUP>(k, check);
+        case kMetricAxis: return mf_tile_kernel_of<kMetricAxis, kRadPacked, SUP>(k, check);
+        case kMetricConst: return mf_tile_kernel_of<kMetricConst, kRadPlanar, SUP>(k, check);
+        default: return mf_tile_kernel_of<kMetricField, kRadPacked, SUP>(k, check);
+    }
 }
 
 }  // namespace
