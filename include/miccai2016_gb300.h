@@ -113,11 +113,11 @@ typedef struct m16_solve_stats {
     double u_ms;           /* out: summed device time of the U launches (time_kernels only) */
     int32_t path;          /* in: M16_PATH_* -- how an iteration is launched */
     int32_t flags;         /* in: M16_BATCH_* options of m16_batch_solve (0 elsewhere) */
-    int32_t blocks_per_sm; /* out (m16_batch_solve): the sweeps' tile shape in use at the end, as the
-                              target blocks per SM its z-chunk was chosen for; in, with
+    int32_t blocks_per_sm; /* out (m16_batch_solve): the sweeps' tile shape in use at the end: 16 is the
+                              default chunk of planes per block, 8 twice and 32 half of it; in, with
                               M16_BATCH_NO_TUNE: 8, 16 or 32 fixes that shape (0: the default) */
-    int32_t pair_launches; /* out (single solve): launches of two iterations that ran */
-    double pair_ms;        /* out (single solve): their summed device time (time_kernels only) */
+    int32_t pair_launches; /* out: launches of two iterations that ran (m16_batch_solve: time_kernels only) */
+    double pair_ms;        /* out: their summed device time (time_kernels only) */
     int32_t pair_zc;       /* out (single solve): planes per block of those launches */
     int32_t reserved;
 } m16_solve_stats;
@@ -212,8 +212,10 @@ size_t m16_batch_workspace_bytes(const m16_batch_volume *vols, int32_t nvol, con
  * residual and stopping rule from params; params->scaling is ignored, each
  * volume carries its own).  iterations and residuals (host, ninst each,
  * optional) receive each instance's iteration count and last residual.
- * stats (host, optional) counts launches and, with time_kernels, the summed
- * device time of the batched flow/label launches.  Synchronizes `stream`.
+ * stats (host, optional) counts launches and, with time_kernels, the launches
+ * of two iterations and their summed device time (pair_launches, pair_ms).
+ * Synchronizes `stream`.  A batch whose double-buffered state (48 bytes per
+ * voxel and instance) is above 128 GiB is solved in cohorts that fit.
  */
 int m16_batch_solve(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst, int32_t ninst,
                     const m16_cut_params *params, int32_t *iterations, double *residuals, void *workspace,
@@ -222,14 +224,14 @@ int m16_batch_solve(const m16_batch_volume *vols, int32_t nvol, const m16_batch_
 /*
  * The same batch as a sequence of steps.  m16_batch_begin prepares the batch
  * on `stream` (descriptors, set-up kernels, the default tile shape, a work
- * list over every group; nothing is synchronised) and returns a handle.
+ * list over every instance; nothing is synchronised) and returns a handle.
  * m16_batch_iterate enqueues `count` iterations (not past num_iter), with a
  * residual check on every iteration index that is a multiple of update, and
  * does nothing else: no synchronisation, allocation or copy, so a caller may
  * capture it into a CUDA graph.  A graph captured from a call that starts at
  * a multiple of update and runs update iterations replays one check interval.
- * Instances stop at their residual bound on the device (their lanes are
- * masked).  m16_batch_end scatters every instance's u to its output, reports
+ * Instances stop at their residual bound on the device.  m16_batch_end
+ * writes every instance's u to its output, reports
  * iterations (at the stop, else the iterations that ran) and the last
  * residuals, and frees the handle; it synchronizes `stream`.  The three calls
  * take the same stream (or the caller orders them).  The workspace
@@ -248,9 +250,9 @@ int m16_batch_end(m16_batch *b, int32_t *iterations, double *residuals, void *st
  * No reference interface: the reference solves one CmfCutQAnisotropicGpu at a
  * time.  A server owns one caller workspace; requests (each its own volume)
  * are admitted while the workspace has room, their inputs are uploaded on a
- * copy stream, and every m16_server_step advances all resident requests by
- * params->update iterations (one residual check each, at the request's own
- * iterations 0, update, 2 update, ...), so a request's iterations, residuals
+ * copy stream, iteration 0 runs at admission, and every m16_server_step
+ * advances all resident requests by params->update iterations (one residual
+ * check each, at the request's own iterations 0, update, 2 update, ...), so a request's iterations, residuals
  * and u are the same as those of m16_maxflow_solve on its inputs alone.  A
  * request retires at the residual bound (or NaN) or at params->num_iter; its
  * u is then copied to the request's host buffer and the memory is reused. */
@@ -283,7 +285,9 @@ typedef struct m16_server_info {
     double gpu_ms;        /* device time of the steps' kernels (CUDA events) */
 } m16_server_info;
 
-/* Workspace bytes a request of d0 x d1 x d2 voxels holds while resident. */
+/* Workspace bytes a request of d0 x d1 x d2 voxels holds while resident (76
+ * instead of 72 per voxel with three different eigenvalues).  A request that
+ * does not fit into an idle server that way is run by slower sweeps in 68. */
 size_t m16_server_request_bytes(int32_t d0, int32_t d1, int32_t d2, int32_t has_alpha);
 
 /* Workspace bytes the server keeps for its tables (the rest holds requests). */
@@ -300,7 +304,8 @@ int m16_server_create(const m16_cut_params *params, int32_t max_slots, int32_t m
  * request has been returned by m16_server_poll. */
 int m16_server_admit(m16_server *s, const m16_serve_request *req, int32_t *admitted);
 
-/* params->update iterations of every resident request, then retirement. */
+/* The iterations up to the next check of every resident request (update of
+ * them; after its last check those that remain), then retirement. */
 int m16_server_step(m16_server *s);
 
 /* Requests whose u has reached the host since the last call: tags,

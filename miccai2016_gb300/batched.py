@@ -46,8 +46,7 @@ class BatchedCut(object):
         with 'volume' (index), 'eigs' (3 constant eigenvalues) and either
         ('weighting', 'decay') or 'alpha' (an array of the volume's shape).
         path is accepted for symmetry with the single solve; the batched
-        engine has one iteration path (flow and label sweeps over groups of
-        four interleaved instances).  graphs=False launches every iteration
+        engine has one iteration path.  graphs=False launches every iteration
         directly instead of replaying CUDA graphs of whole check intervals;
         tune=False keeps the default tile shape instead of timing the
         candidates on the first check intervals, or the shape of
@@ -213,8 +212,8 @@ class BatchSteps(object):
 
 def _main(argv=None):
     """Timing of one batch: python -m miccai2016_gb300.batched --side 128 --instances 64
-    Prints one JSON line with the batch's solves/s and the per-launch device
-    time of the batched flow and label sweeps (CUDA events)."""
+    Prints one JSON line with the batch's voxel-iterations/s and the device
+    time of its launches of two iterations (CUDA events)."""
     import argparse
     import json
     import time
@@ -252,16 +251,12 @@ def _main(argv=None):
     n = int(np.prod(shape))
     out = dict(side=a.side, instances=a.instances, iters=a.iters, graphs=not a.no_graphs, wall_s=dt,
                voxel_iterations_per_s=a.instances * a.iters * n / dt)
-    if a.time_kernels and st.p_launches:
-        pm = (st.p_ms + st.u_ms) / st.p_launches
-        # state bytes per instance and voxel-iteration: the flow sweep reads
-        # tmp 4 + hp 12 and writes hp 12, the label sweep reads hp 12 + pt 4 +
-        # u 4 and writes pt 4 + u 4 + tmp 4 = 60 B.  The volume's shared fields
-        # (read once per group of four) are not counted.
-        sb = 60.0
-        out.update(iteration_ms=pm, state_bytes=sb, state_gbs=sb * a.instances * n / (pm * 1e-3) / 1e9)
-        if st.u_launches:
-            out.update(flow_ms=st.p_ms / st.p_launches, label_ms=st.u_ms / st.u_launches)
+    if a.time_kernels and st.pair_launches:
+        pm = st.pair_ms / st.pair_launches
+        # state bytes per instance and voxel of two iterations: hp 12, tmp 4,
+        # u 4 and pt 4 read and written.  The volume's shared fields are not
+        # counted.
+        out.update(pair_ms=pm, state_gbs=48.0 * a.instances * n / (pm * 1e-3) / 1e9)
     print(json.dumps(out))
 
 

@@ -1,7 +1,7 @@
 // batch_kernels.cuh -- device side of the batched ATV max-flow: descriptors,
-// set-up kernels, the flow / label sweeps over a work list of (group, tile)
-// items, the per-instance residual check and the scatter of u.  Included by
-// batched.cu (m16_batch_solve: a fixed batch run to completion) and serve.cu
+// set-up kernels, the sweeps over a work list of (instance, tile) items, the
+// per-instance residual check and the output of u.  Included by batched.cu
+// (m16_batch_solve: a fixed batch run to completion) and serve.cu
 // (m16_server_*: requests admitted and retired while others iterate).
 //
 // The reference runs its (weighting, decay) grid search as one
@@ -9,32 +9,32 @@
 // (src/phantom_experiment.py:350-368), each with three launches per iteration
 // and a blocking residual read every `update` iterations.  Here a batch of
 // instances -- any mix of volumes, weightings, decays and eigenvalue sets --
-// advances together: every flow (P) and label (U) launch covers all active
-// instances, the residual check of every instance is one block of one launch,
-// and an instance stops on its own at its threshold.
+// advances together: a launch runs two iterations (tile_sweep.cuh) of every
+// active instance of one kind, the residual check of every instance is one
+// block of one launch, and an instance stops on its own at its threshold.
 //
-// Layout.  Instances of one volume with the same eigenvalues (and the same
-// kind of alpha) form groups of kLanes = 4; a group's state is interleaved,
-// one float4 per voxel and field (lane = instance), so one 16-byte load or
-// store serves four solves and a warp moves 512 contiguous bytes per field.
-// The volume's quaternions, |grad I|^2 and capacities are read once per voxel
-// for the whole group and the rotation is built once.  The projection radius
-// of a lane is its alpha field (gathered into an interleaved field at set-up)
-// or w * exp(-|grad I|^2 / decay^2) (phantom_experiment.py:359) computed in
-// the flow sweep, so per voxel and instance only the state streams from HBM:
-// flow reads tmp 4 + hp 12 and writes hp 12, labels read hp 12 + p_t 4 + u 4
-// and write p_t 4 + u 4 + tmp 4 -- 60 B per voxel-iteration.
+// Layout.  An instance has its own state, double-buffered.  The direction
+// field with |grad I|^2, the capacities and, for isotropic and three-valued
+// metrics, |grad I|^2 alone belong to the volume; the work list puts the
+// instances of a volume side by side for every tile, so these fields come from
+// L2 for all but the first of them.  The projection radius is an instance's
+// own alpha field or w * exp(-|grad I|^2 / decay^2) (phantom_experiment.py:359)
+// computed in the sweep.
 //
-// Instances whose volume is shared by fewer than three others of the same
-// kind (ragged batches, served requests) form one-lane groups instead: plain
-// float fields and the single solve's z-batched sweep bodies (sweeps.cuh),
-// so no padding lanes stream.
+// An instance's state word holds its stop flag and which buffer is current.
+// Within a run of launches between two checks the buffers alternate by the
+// launch's number; the check that ends the run stores the buffer it ends in,
+// so captured launches can be replayed.
 //
-// Stopping.  The check kernel sets a lane's bit in its group's stop mask; the
-// label sweep then keeps that lane's u (the solve's result) unchanged, blocks
-// of a group whose lanes have all stopped return at once, and the work list
-// drops finished groups.  At the end u is scattered out of the interleaved
-// field into each instance's output array.
+// Measured on GB300: 16 grid points at 128^3, anisotropic and isotropic (32
+// instances), 358 -> 154 ms against groups of four interleaved instances in a
+// flow and a label launch per iteration; eight uneven volumes 46.4 -> 21.6 ms;
+// ten served requests 112 -> 51.6 ms.  Bound by HBM: 48 bytes of state per
+// voxel and two iterations (tile_sweep.cuh).
+//
+// The compact sweeps at the end (one buffer, planar fields, a flow and a label
+// launch per iteration) take the instances whose double-buffered state does
+// not fit.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -42,20 +42,19 @@
 #include <float.h>
 
 #include <algorithm>
-#include <map>
-#include <tuple>
 #include <vector>
 
 #include "common.cuh"
 #include "sweeps.cuh"
+#include "tile_sweep.cuh"
 
 namespace m16 {
 namespace {
 
 constexpr int kBX = 32, kBY = 8, kTile = kBX * kBY;
-constexpr int kLanes = 4;     // instances per group: one float4 per voxel and field
-constexpr int kFields = 6;    // hp0 hp1 hp2 pt tmp u (+ alpha for groups with alpha fields)
-constexpr unsigned kAllLanes = (1u << kLanes) - 1u;
+constexpr int kSetupBlocks = 4 * kSMs;
+
+constexpr unsigned kStopped = 1u, kBuffer = 2u;   // bits of an instance's state word
 
 struct InstCtrl {
     int stopped;
@@ -65,71 +64,33 @@ struct InstCtrl {
     double resid;   // last checked residual
 };
 
-struct VolDev {
-    int d0, d1, d2, zc, tx, ty, tz, pad;
-    float rcc, rs0, rs1, rs2, ss0, ss1, ss2, denom;
-    const float4 *q4;
-    const float *grad2, *cs, *ct;
-    int64_t n;
-};
-
-struct GroupDev {
-    int64_t part_off;        // float4 index of the group's first partial sum
-    int vol, nparts, has_alpha;
-    int lanes, pad0, pad1, pad2;   // 4: interleaved float4 fields; 1: plain float fields
-    float4 w, nid2;          // per lane: alpha = w * exp(nid2 * |grad I|^2), nid2 = -1 / decay^2
-    float sq0, sq1, sq2, isq0, isq1, isq2;
-    void *state;             // kFields (+1 for 4-lane alpha groups) slabs of `slab` elements
-    int64_t slab;            // elements (float4 or float) per slab
-    const float *alpha1;     // one-lane groups: the instance's own alpha field, or NULL
-};
-
+// what the check and the output need of an instance
 struct InstDev {
-    int group, lane;
+    int64_t n;
+    int64_t part_off;        // float index of its first partial sum
+    int nparts, d2;
+    float rcc;
+    const float2 *u2[2];     // padded (tile sweeps), or null:
+    const float *u1;         // the compact sweeps' u
     float *u_out;
-    const float *alpha;
 };
 
-// z-slices per block: enough blocks for `blocks_per_sm` (by default
-// M16_BATCH_BLOCKS_PER_SM) per SM over the volume's groups (many short blocks
-// keep the last wave short), at most 32
-#ifndef M16_BATCH_BLOCKS_PER_SM
-#define M16_BATCH_BLOCKS_PER_SM 16
-#endif
-// resident blocks per SM of the four-lane sweeps: 4 caps them at 64
-// registers (a few bytes spill to L1); measured on GB300 (424 instances at
-// 128^3) one iteration takes 8.64 ms against 9.09 ms at 3 and 10.21 ms at 2
-#ifndef M16_BATCH_MINB
-#define M16_BATCH_MINB 4
-#endif
-inline int batch_zc(int d0, int d1, int d2, int ngroups_of_volume, int blocks_per_sm = M16_BATCH_BLOCKS_PER_SM)
-{
-    const int64_t cols = div_up(d2, kBX) * div_up(d1, kBY);
-    int64_t zc = (int64_t)d0 * cols * std::max(ngroups_of_volume, 1) / ((int64_t)blocks_per_sm * kSMs);
-    zc = std::max<int64_t>(1, std::min<int64_t>(32, zc));
-    return (int)zc;
-}
+// an instance of the tile sweeps
+struct TileDev {
+    TileView V;              // all but the buffers
+    const CUtensorMap *mh[2], *mu[2];
+    float4 *h[2];
+    float2 *u[2];
+    int64_t part_off, rows;
+    int nx, ny, zc;
+    // set-up inputs
+    const float *img, *cs, *ct, *alpha, *denom;
+    float *rad;              // its own padded radius field (alpha instances), or null
+};
 
-// One z-chunk for every volume of a launch: the launch covers the tiles of
-// all its groups, so the target number of blocks applies to their sum
-// (total_column_slices = sum over groups of d0 x the volume's 32 x 8 columns).
-#ifndef M16_BATCH_ZC_ROUND
-#define M16_BATCH_ZC_ROUND 4
-#endif
-inline int batch_zc_total(int64_t total_column_slices, int blocks_per_sm = M16_BATCH_BLOCKS_PER_SM)
-{
-    int64_t zc = total_column_slices / ((int64_t)blocks_per_sm * kSMs);
-    zc = std::max<int64_t>(1, std::min<int64_t>(32, zc));
-    if (zc >= M16_BATCH_ZC_ROUND) zc = zc / M16_BATCH_ZC_ROUND * M16_BATCH_ZC_ROUND;
-    return (int)zc;
-}
-
-inline int64_t column_slices(int d0, int d1, int d2) { return (int64_t)d0 * div_up(d2, kBX) * div_up(d1, kBY); }
-
-__device__ __forceinline__ float lane_of(const float4 &v, int l)
-{
-    return l == 0 ? v.x : (l == 1 ? v.y : (l == 2 ? v.z : v.w));
-}
+// kinds of launches: the tile sweeps' instantiations, then the compact sweeps
+enum BatchKind { kAxisPacked = 0, kAxisPlanar, kIsoPlanar, kConstPlanar, kTileKinds, kCompactAlpha = kTileKinds,
+                 kCompactExp, kKinds };
 
 // ---- initialisation ---------------------------------------------------------
 
@@ -157,17 +118,259 @@ __global__ void bt_max_kernel(const float *__restrict__ img, int64_t n, float *_
     }
 }
 
-__global__ void bt_denom_kernel(const float *__restrict__ part, int nparts, VolDev *vol)
+// *denom = np.max(img) + np.finfo(float32).tiny (one block)
+__global__ void __launch_bounds__(256) bt_denom_kernel(const float *__restrict__ part, int nparts, float *denom)
 {
-    if (threadIdx.x != 0) return;
+    __shared__ float s[256];
+    __shared__ int snan;
+    if (threadIdx.x == 0) snan = 0;
+    __syncthreads();
     float m = -INFINITY;
-    bool nan = false;
-    for (int k = 0; k < nparts; ++k) {
+    for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
         const float v = part[k];
-        if (v != v) nan = true; else m = fmaxf(m, v);
+        if (v != v) snan = 1; else m = fmaxf(m, v);
     }
-    vol->denom = (nan ? NAN : m) + FLT_MIN;   // np.max(img) + np.finfo(float32).tiny
+    s[threadIdx.x] = m;
+    __syncthreads();
+    for (int w = blockDim.x >> 1; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) s[threadIdx.x] = fmaxf(s[threadIdx.x], s[threadIdx.x + w]);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *denom = (snan ? NAN : s[0]) + FLT_MIN;
 }
+
+// the volume's padded fields: caps and, where given, the direction of each
+// axis with `value` (|grad I|^2 or alpha), the quaternion, and value alone
+struct VolumeFields {
+    float2 *caps;
+    float4 *dir[3], *q4;
+    float *rad;
+};
+
+__global__ void bt_volume_kernel(const float *__restrict__ quat3, const float *__restrict__ value,
+                                 const float *__restrict__ cs, const float *__restrict__ ct, int d2, int64_t rows,
+                                 VolumeFields F)
+{
+    const int pitch = tile_pitch(d2);
+    const int64_t np = rows * pitch;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < np; o += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = o / pitch;
+        const int x = (int)(o - row * pitch);
+        const bool in = x < d2;   // the padding is never part of a result; kept finite
+        const int64_t i = row * d2 + (in ? x : 0);
+        const float v = in && value ? value[i] : 0.f;
+        F.caps[o] = in ? make_float2(cs[i], ct[i]) : make_float2(0.f, 0.f);
+        for (int k = 0; k < 3; ++k)
+            if (F.dir[k]) F.dir[k][o] = tile_direction(quat3 + 3 * i, k, v);
+        if (F.q4) F.q4[o] = qexpand(quat3[3 * i], quat3[3 * i + 1], quat3[3 * i + 2]);
+        if (F.rad) F.rad[o] = v;
+    }
+}
+
+// every instance (blockIdx.y): h4 = (0, 0, 0, -u rcc), u2 = (u, fmin(cs, ct))
+// with u = img / denom (continuous_cut_anisotropic_gpu.py:276-289) in buffer 0,
+// and its own radius field
+__global__ void bt_state_kernel(const TileDev *tiles, int first)
+{
+    const TileDev &T = tiles[first + blockIdx.y];
+    const float denom = *T.denom, rcc = T.V.rcc;
+    const int d2 = T.V.d2, pitch = T.V.pitch;
+    const int64_t np = T.rows * pitch;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < np; o += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = o / pitch;
+        const int x = (int)(o - row * pitch);
+        const bool in = x < d2;
+        const int64_t i = row * d2 + (in ? x : 0);
+        const float u = in ? T.img[i] / denom : 0.f;
+        T.h[0][o] = make_float4(0.f, 0.f, 0.f, -(u * rcc));
+        T.u[0][o] = make_float2(u, in ? fminf(T.cs[i], T.ct[i]) : 0.f);
+        if (T.rad) T.rad[o] = in ? T.alpha[i] : 0.f;
+    }
+}
+
+// u of every instance (blockIdx.y) into its output; flip: the buffer is the
+// other one than the state word says
+__global__ void bt_result_kernel(const InstDev *insts, const unsigned *state, int first, int flip)
+{
+    const InstDev &I = insts[first + blockIdx.y];
+    const int b = ((state[first + blockIdx.y] & kBuffer) ? 1 : 0) ^ flip;
+    const float2 *u2 = I.u2[b];
+    const int pitch = tile_pitch(I.d2);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < I.n; i += (int64_t)gridDim.x * blockDim.x)
+        I.u_out[i] = u2 ? u2[i / I.d2 * pitch + i % I.d2].x : I.u1[i];
+}
+
+// ---- the tile sweeps ----------------------------------------------------------
+
+// K iterations of the work items' tiles; work == NULL: block b is tile b of
+// instance `first`.  The launch reads the current buffer, or with `odd` (an odd
+// launch since the state word was set) the other one.
+template <int K, int METRIC, int ASRC, bool CHECK>
+__global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) bt_tile_kernel(const int2 *__restrict__ work,
+                                                                                  int first, const TileDev *tiles,
+                                                                                  const unsigned *__restrict__ state,
+                                                                                  float *__restrict__ partials,
+                                                                                  int odd)
+{
+    extern __shared__ __align__(128) unsigned char tile_mem[];
+    __shared__ float red[32];
+    TileMem<METRIC, ASRC> &M = *reinterpret_cast<TileMem<METRIC, ASRC> *>(tile_mem);
+    tile_init(M);
+    pdl_wait();
+    pdl_launch_next();
+    const int2 wk = work ? work[blockIdx.x] : make_int2(first, (int)blockIdx.x);
+    const unsigned s = __ldcg(state + wk.x);
+    if (s & kStopped) return;   // uniform over the block
+    const int b = ((s & kBuffer) ? 1 : 0) ^ odd;
+    const TileDev &T = tiles[wk.x];
+    TileView V = T.V;
+    V.mh = T.mh[b];
+    V.mu = T.mu[b];
+    V.ho = T.h[1 - b];
+    V.uo = T.u[1 - b];
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        tile_acquire(V.mh);
+        tile_acquire(V.mu);
+        tile_acquire(V.mcaps);
+        if (METRIC != kMetricIso) tile_acquire(V.mdir);
+        if (ASRC == kRadPlanar) tile_acquire(V.mrad);
+    }
+    const int nx = T.nx, ny = T.ny, zc = T.zc;
+    const int bx = wk.y % nx, t = wk.y / nx, by = t % ny, za = t / ny * zc;
+    float acc[2] = {0.f, 0.f};
+    tile_sweep<K, METRIC, ASRC, true, false, CHECK>(V, M, bx, by, za, min(za + zc, V.d0), acc);
+    if (CHECK) {
+        const float sum = block_sum(acc[K - 1], red);
+        if (threadIdx.x == 0 && threadIdx.y == 0) partials[T.part_off + wk.y] = sum;
+    }
+}
+
+typedef void (*BatchTileKernel)(const int2 *, int, const TileDev *, const unsigned *, float *, int);
+
+struct BatchTileLaunch {
+    BatchTileKernel kernel;
+    size_t smem;
+};
+
+template <int METRIC, int ASRC>
+BatchTileLaunch batch_tile_kernel(int k, bool check)
+{
+    BatchTileLaunch L;
+    L.smem = sizeof(TileMem<METRIC, ASRC>);
+    if (k == 2) L.kernel = check ? bt_tile_kernel<2, METRIC, ASRC, true> : bt_tile_kernel<2, METRIC, ASRC, false>;
+    else L.kernel = check ? bt_tile_kernel<1, METRIC, ASRC, true> : bt_tile_kernel<1, METRIC, ASRC, false>;
+    return L;
+}
+
+inline BatchTileLaunch batch_tile_pick(int kind, int k, bool check)
+{
+    switch (kind) {
+        case kAxisPacked: return batch_tile_kernel<kMetricAxis, kRadPacked>(k, check);
+        case kAxisPlanar: return batch_tile_kernel<kMetricAxis, kRadPlanar>(k, check);
+        case kIsoPlanar: return batch_tile_kernel<kMetricIso, kRadPlanar>(k, check);
+        default: return batch_tile_kernel<kMetricConst, kRadPlanar>(k, check);
+    }
+}
+
+// once per device and call, before any launch (not while capturing)
+inline cudaError_t batch_tile_prepare(int kind)
+{
+    for (int k = 1; k <= 2; ++k)
+        for (int c = 0; c < 2; ++c) {
+            const BatchTileLaunch L = batch_tile_pick(kind, k, c != 0);
+            const cudaError_t e =
+                cudaFuncSetAttribute(L.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+// TileView constants of a volume (scaling sc) under the solve's parameters
+inline void tile_view(TileView &V, int d0, int d1, int d2, const double *sc, const m16_cut_params &p)
+{
+    const double smin = fmin(sc[0], fmin(sc[1], sc[2]));
+    const double rcc = 1.0 / (p.cc * (smin * smin));
+    V.d0 = d0; V.d1 = d1; V.d2 = d2; V.pitch = tile_pitch(d2);
+    V.ss0 = (float)(p.steps / sc[0] * (smin * smin));
+    V.ss1 = (float)(p.steps / sc[1] * (smin * smin));
+    V.ss2 = (float)(p.steps / sc[2] * (smin * smin));
+    V.rs0 = (float)(1.0 / sc[0]); V.rs1 = (float)(1.0 / sc[1]); V.rs2 = (float)(1.0 / sc[2]);
+    V.rcc = (float)rcc;
+    V.ircc = (float)(1.0 / rcc);
+}
+
+// one block per instance: residual = sum of its partial sums / (N * rcc); below
+// the bound (or NaN) the instance stops.  Every instance is checked at its own
+// iterations 0, update, 2 update, ..., so the n-th check (from 0) follows
+// iteration n * update and a stop there counts n * update + 1 iterations,
+// wherever the instance joined the batch.  flip: the run of launches that the
+// check ends was odd, so the other buffer is the current one now.
+__global__ void bt_check_kernel(const InstDev *insts, InstCtrl *ctrl, unsigned *state,
+                                const float *__restrict__ partials, double bound, int update, int flip,
+                                const int *__restrict__ list, int first)
+{
+    pdl_wait();
+    pdl_launch_next();
+    __shared__ double s[256];
+    const int inst = list ? list[blockIdx.x] : first + (int)blockIdx.x;   // list: the instances to check
+    const unsigned word = __ldcg(state + inst);
+    if (word & kStopped) return;
+    const InstDev &I = insts[inst];
+    InstCtrl &C = ctrl[inst];
+    const float *p = partials + I.part_off;
+    double acc = 0.0;
+    for (int k = threadIdx.x; k < I.nparts; k += blockDim.x) acc += (double)p[k];
+    s[threadIdx.x] = acc;
+    __syncthreads();
+    for (int w = blockDim.x >> 1; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double err = s[0] / ((double)I.n * (double)I.rcc);
+        C.resid = err;
+        const int n = C.n_checks;
+        C.n_checks = n + 1;
+        unsigned w = flip ? word ^ kBuffer : word;
+        if (isnan(err) || err < bound) {
+            C.stopped = 1;
+            C.iterations = n * update + 1;
+            w |= kStopped;
+        }
+        state[inst] = w;
+    }
+}
+
+// the end of an odd run of launches without a check
+__global__ void bt_flip_kernel(unsigned *state, int n)
+{
+    pdl_wait();
+    pdl_launch_next();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && !(state[i] & kStopped)) state[i] ^= kBuffer;
+}
+
+// ---- the compact sweeps: the single solve's two sweeps over the work list ------
+
+struct VolDev {
+    int d0, d1, d2, zc, tx, ty, tz, pad;
+    float rcc, rs0, rs1, rs2, ss0, ss1, ss2;
+    const float4 *q4;
+    const float *grad2, *cs, *ct;
+};
+
+struct GroupDev {
+    int vol, pad;
+    int64_t part_off;
+    float w, nid2;           // radius = w * exp(nid2 * |grad I|^2), nid2 = -1 / decay^2
+    float sq0, sq1, sq2, isq0, isq1, isq2;
+    float *state;            // hp0 hp1 hp2 pt tmp u: slabs of `slab` floats
+    int64_t slab;
+    const float *alpha;      // the instance's own radius, or NULL
+    const float *img, *denom;
+};
+
+constexpr int kFields = 6;
 
 __global__ void bt_expand_kernel(const float *__restrict__ quat3, float4 *__restrict__ q4, int64_t n)
 {
@@ -175,67 +378,23 @@ __global__ void bt_expand_kernel(const float *__restrict__ quat3, float4 *__rest
         q4[i] = qexpand(quat3[3 * i], quat3[3 * i + 1], quat3[3 * i + 2]);
 }
 
-// every lane of a group: hp = 0, p_t = fmin(cs, ct), u = img / denom,
-// tmp = -u * rcc (continuous_cut_anisotropic_gpu.py:276-289)
-__global__ void bt_init_group_kernel(const float *__restrict__ img, const VolDev *vols, const GroupDev *groups, int g)
+__global__ void bt1_state_kernel(const VolDev *vols, const GroupDev *groups, int first)
 {
-    const GroupDev &G = groups[g];
+    const GroupDev &G = groups[first + blockIdx.y];
     const VolDev &V = vols[G.vol];
-    const float denom = V.denom;
-    const int64_t S = G.slab;
-    if (G.lanes == 1) {
-        float *st1 = (float *)G.state;
-        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V.n;
-             i += (int64_t)gridDim.x * blockDim.x) {
-            const float ui = img[i] / denom;
-            st1[i] = 0.f;
-            st1[S + i] = 0.f;
-            st1[2 * S + i] = 0.f;
-            st1[3 * S + i] = fminf(V.cs[i], V.ct[i]);
-            st1[4 * S + i] = -(ui * V.rcc);
-            st1[5 * S + i] = ui;
-        }
-        return;
-    }
-    float4 *st = (float4 *)G.state;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float ptv = fminf(V.cs[i], V.ct[i]);
-        const float ui = img[i] / denom;
-        const float ti = -(ui * V.rcc);
-        st[i] = zero;
-        st[S + i] = zero;
-        st[2 * S + i] = zero;
-        st[3 * S + i] = make_float4(ptv, ptv, ptv, ptv);
-        st[4 * S + i] = make_float4(ti, ti, ti, ti);
-        st[5 * S + i] = make_float4(ui, ui, ui, ui);
+    const float denom = *G.denom;
+    const int64_t S = G.slab, n = (int64_t)V.d0 * V.d1 * V.d2;
+    float *st = G.state;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float ui = G.img[i] / denom;
+        st[i] = 0.f;
+        st[S + i] = 0.f;
+        st[2 * S + i] = 0.f;
+        st[3 * S + i] = fminf(V.cs[i], V.ct[i]);
+        st[4 * S + i] = -(ui * V.rcc);
+        st[5 * S + i] = ui;
     }
 }
-
-// interleave the lanes' alpha fields (absent lanes: 0)
-__global__ void bt_gather_alpha_kernel(const GroupDev *groups, int g, const float *a0, const float *a1,
-                                       const float *a2, const float *a3, int64_t n)
-{
-    const GroupDev &G = groups[g];
-    float4 *al = (float4 *)G.state + kFields * G.slab;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        al[i] = make_float4(a0 ? a0[i] : 0.f, a1 ? a1[i] : 0.f, a2 ? a2[i] : 0.f, a3 ? a3[i] : 0.f);
-}
-
-// u of one instance out of its group's interleaved field
-__global__ void bt_scatter_u_kernel(const GroupDev *groups, const InstDev *insts, int inst, int64_t n)
-{
-    const InstDev &I = insts[inst];
-    const GroupDev &G = groups[I.group];
-    const int L = G.lanes;
-    const float *u = (const float *)G.state + 5 * G.slab * L;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        I.u_out[i] = u[L * i + I.lane];
-}
-
-// ---- the sweeps ---------------------------------------------------------------
-// A work item is (group, tile); a block of 32 x 8 threads walks the tile's
-// z-chunk, one (y, x) column per thread, all four lanes of the group per voxel.
 
 __device__ __forceinline__ void decode_tile(const VolDev &V, int tile, int &bx, int &by, int &bz)
 {
@@ -244,222 +403,38 @@ __device__ __forceinline__ void decode_tile(const VolDev &V, int tile, int &bx, 
     bz = tile / (V.tx * V.ty);
 }
 
-// P (update_qp.cl:150-232) for the four lanes of a group
-template <bool ALPHA_ARR>
-__global__ void __launch_bounds__(kTile, M16_BATCH_MINB) bt_flow_kernel(const int2 *__restrict__ work,
-                                                                       const VolDev *vols, const GroupDev *groups,
-                                                                       const unsigned *__restrict__ gmask)
-{
-    pdl_wait();
-    pdl_launch_next();
-    const int2 wk = work[blockIdx.x];
-    if (__ldcg(gmask + wk.x) == kAllLanes) return;
-    const GroupDev &G = groups[wk.x];
-    const VolDev &V = vols[G.vol];
-    int bx, by, bz;
-    decode_tile(V, wk.y, bx, by, bz);
-    const int d0 = V.d0, d1 = V.d1, d2 = V.d2;
-    const int x = bx * kBX + threadIdx.x, y = by * kBY + threadIdx.y;
-    const int z0 = bz * V.zc, z1 = min(z0 + V.zc, d0);
-    if (x >= d2 || y >= d1) return;
-    const int s0 = d1 * d2;
-    const bool yin = y < d1 - 1, xin = x < d2 - 1;
-    const float ss0 = V.ss0, ss1 = V.ss1, ss2 = V.ss2;
-    const float sq[3] = {G.sq0, G.sq1, G.sq2};
-    const float isq[3] = {G.isq0, G.isq1, G.isq2};
-    const float4 w4 = G.w, n4 = G.nid2;
-    const int64_t S = G.slab;
-    float4 *__restrict__ hp0 = (float4 *)G.state;
-    float4 *__restrict__ hp1 = hp0 + S;
-    float4 *__restrict__ hp2 = hp1 + S;
-    const float4 *__restrict__ tmp = hp0 + 4 * S;
-    const float4 *__restrict__ al4 = hp0 + kFields * S;
-    const float4 *__restrict__ q4 = V.q4;
-    const float *__restrict__ grad2 = V.grad2;
-    for (int z = z0; z < z1; ++z) {
-        const int i = (z * d1 + y) * d2 + x;
-        const bool zin = z < d0 - 1;
-        const float4 q = __ldg(q4 + i);
-        float4 a4;
-        float g2 = 0.f;
-        if (ALPHA_ARR) a4 = __ldg(al4 + i);
-        else g2 = __ldg(grad2 + i);
-        const float4 tc = __ldg(tmp + i);
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 tz = zin ? __ldg(tmp + i + s0) : zero;
-        const float4 ty = yin ? __ldg(tmp + i + d2) : zero;
-        const float4 tx = xin ? __ldg(tmp + i + 1) : zero;
-        const float4 h0 = hp0[i], h1 = hp1[i], h2 = hp2[i];
-        const Rot R = quat2rot(q);
-        float o0[kLanes], o1[kLanes], o2[kLanes];
-#pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-            const float c = lane_of(tc, l);
-            const float3 gr = make_float3(zin ? (lane_of(tz, l) - c) * ss0 : 0.f,
-                                          yin ? (lane_of(ty, l) - c) * ss1 : 0.f,
-                                          xin ? (lane_of(tx, l) - c) * ss2 : 0.f);
-            const float rad = ALPHA_ARR ? lane_of(a4, l) : lane_of(w4, l) * expf(lane_of(n4, l) * g2);
-            const float3 rg = rot_t(R, gr);
-            const float3 rh = rot_t(R, make_float3(lane_of(h0, l), lane_of(h1, l), lane_of(h2, l)));
-            float3 p = make_float3(rh.x * isq[0] + rg.x * sq[0], rh.y * isq[1] + rg.y * sq[1],
-                                   rh.z * isq[2] + rg.z * sq[2]);
-            const float nrm = sqrtf(p.x * p.x + p.y * p.y + p.z * p.z);
-            const float sc = nrm > rad ? rad / nrm : 1.f;
-            p = make_float3(p.x * sc * sq[0], p.y * sc * sq[1], p.z * sc * sq[2]);
-            const float3 h = rot(R, p);
-            o0[l] = h.x;
-            o1[l] = h.y;
-            o2[l] = h.z;
-        }
-        hp0[i] = make_float4(o0[0], o0[1], o0[2], o0[3]);
-        hp1[i] = make_float4(o1[0], o1[1], o1[2], o1[3]);
-        hp2[i] = make_float4(o2[0], o2[1], o2[2], o2[3]);
-    }
-}
-
-// U with update_tmp fused (update_qp.cl:241-300, :311-316) for the four lanes
-// of a group; a stopped lane keeps its u.  On check iterations the block's
-// per-lane sum of |err| goes to partials[part_off + tile] (fixed order).
-template <bool CHECK>
-__global__ void __launch_bounds__(kTile, M16_BATCH_MINB) bt_label_kernel(const int2 *__restrict__ work,
-                                                                        const VolDev *vols, const GroupDev *groups,
-                                                                        const unsigned *__restrict__ gmask,
-                                                                        float4 *__restrict__ partials)
-{
-    pdl_wait();
-    pdl_launch_next();
-    __shared__ float4 red[kTile / 32];
-    const int2 wk = work[blockIdx.x];
-    const unsigned stopped = __ldcg(gmask + wk.x);
-    if (stopped == kAllLanes) return;   // uniform over the block
-    const GroupDev &G = groups[wk.x];
-    const VolDev &V = vols[G.vol];
-    int bx, by, bz;
-    decode_tile(V, wk.y, bx, by, bz);
-    const int d0 = V.d0, d1 = V.d1, d2 = V.d2;
-    const int x = bx * kBX + threadIdx.x, y = by * kBY + threadIdx.y;
-    const int z0 = bz * V.zc, z1 = min(z0 + V.zc, d0);
-    float acc[kLanes] = {0.f, 0.f, 0.f, 0.f};
-    if (x < d2 && y < d1) {
-        const int s0 = d1 * d2;
-        const bool ylo = y > 0, xlo = x > 0, yhi = y < d1 - 1, xhi = x < d2 - 1;
-        const float rcc = V.rcc, rs0 = V.rs0, rs1 = V.rs1, rs2 = V.rs2;
-        const int64_t S = G.slab;
-        float4 *const st = (float4 *)G.state;
-        const float4 *__restrict__ hp0 = st;
-        const float4 *__restrict__ hp1 = hp0 + S;
-        const float4 *__restrict__ hp2 = hp1 + S;
-        float4 *__restrict__ ptp = st + 3 * S;
-        float4 *__restrict__ tmp = st + 4 * S;
-        float4 *__restrict__ up = st + 5 * S;
-        const float *__restrict__ csp = V.cs;
-        const float *__restrict__ ctp = V.ct;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int z = z0; z < z1; ++z) {
-            const int i = (z * d1 + y) * d2 + x;
-            const float4 h0 = __ldg(hp0 + i), h1 = __ldg(hp1 + i), h2 = __ldg(hp2 + i);
-            const float4 h0m = z > 0 ? __ldg(hp0 + i - s0) : zero;
-            const float4 h1m = ylo ? __ldg(hp1 + i - d2) : zero;
-            const float4 h2m = xlo ? __ldg(hp2 + i - 1) : zero;
-            const float4 uo = up[i], pto = ptp[i];
-            const float csv = __ldg(csp + i), ctv = __ldg(ctp + i);
-            const bool zhi = z < d0 - 1;
-            float on[kLanes], op[kLanes], ot[kLanes];
-#pragma unroll
-            for (int l = 0; l < kLanes; ++l) {
-                const float div = ((zhi ? lane_of(h0, l) : 0.f) - lane_of(h0m, l)) * rs0 +
-                                  ((yhi ? lane_of(h1, l) : 0.f) - lane_of(h1m, l)) * rs1 +
-                                  ((xhi ? lane_of(h2, l) : 0.f) - lane_of(h2m, l)) * rs2;
-                const float u0 = lane_of(uo, l);
-                const float psx = div + lane_of(pto, l) - rcc * (u0 - 1.f);
-                const float ps = csv < psx ? csv : psx;
-                const float ptx = -div + ps + rcc * u0;
-                const float ptn = ctv < ptx ? ctv : ptx;
-                const float err = div - ps + ptn;
-                const float un = u0 - err / rcc;
-                op[l] = ptn;
-                on[l] = (stopped >> l) & 1u ? u0 : un;
-                ot[l] = err - un * rcc;
-                if (CHECK) acc[l] += fabsf(err);
-            }
-            ptp[i] = make_float4(op[0], op[1], op[2], op[3]);
-            up[i] = make_float4(on[0], on[1], on[2], on[3]);
-            tmp[i] = make_float4(ot[0], ot[1], ot[2], ot[3]);
-        }
-    }
-    if (CHECK) {
-        const int tid = threadIdx.x + kBX * threadIdx.y;
-#pragma unroll
-        for (int l = 0; l < kLanes; ++l)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[l] += __shfl_down_sync(0xffffffffu, acc[l], o);
-        if ((tid & 31) == 0) red[tid >> 5] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        __syncthreads();
-        if (tid == 0) {
-            float4 s = red[0];
-            for (int w = 1; w < kTile / 32; ++w) {
-                s.x += red[w].x; s.y += red[w].y; s.z += red[w].z; s.w += red[w].w;
-            }
-            partials[G.part_off + wk.y] = s;
-        }
-    }
-}
-
-// ---- one-lane groups: the single solve's sweep bodies over the work list ----
-// resident blocks per SM of the one-lane sweeps: 4 (64 registers) measured
-// fastest on GB300 (the 12-volume ragged batch: 0.91x -> 1.01x its plain solves)
-#ifndef M16_BATCH1_MINB
-#define M16_BATCH1_MINB 4
-#endif
-// z-slices whose loads the one-lane flow / label sweeps issue together, and
-// whether the flow sweep reads its view (the descriptor values) from shared
-// memory.  Measured on GB300 for one 256^3 instance of 1000 iterations (with
-// an alpha field in brackets), the single solve's own sweeps taking 232 ms:
-//   view in registers: flow 1 / label 4 259 (257) ms, flow 2 / label 4 264
-//   (285), flow 1 / label 2 293 (291), flow 2 / label 2 297 (319);
-//   flow view in shared memory, flow 2 / label 4: 245 (243) ms; both views in
-//   shared memory, flow 2 / label 2: 258 (256).
-#ifndef M16_BATCH1_FZB
-#define M16_BATCH1_FZB 2
-#endif
-#ifndef M16_BATCH1_UZB
-#define M16_BATCH1_UZB M16_MF_UZB
-#endif
-// bit 1: the one-lane flow sweep reads its view from shared memory, bit 2:
-// the label sweep does
-#ifndef M16_BATCH1_SMEM_VIEW
-#define M16_BATCH1_SMEM_VIEW 1
-#endif
+// resident blocks per SM of the compact sweeps: 4 (64 registers) measured
+// fastest on GB300
+constexpr int kCompactBlocks = 4;
 
 template <int ALPHA>
-__global__ void __launch_bounds__(kTile, M16_BATCH1_MINB) bt1_flow_kernel(const int2 *__restrict__ work,
-                                                                         const VolDev *vols, const GroupDev *groups,
-                                                                         const unsigned *__restrict__ gmask)
+__global__ void __launch_bounds__(kTile, kCompactBlocks) bt1_flow_kernel(const int2 *__restrict__ work, int first,
+                                                                        const VolDev *vols, const GroupDev *groups,
+                                                                        const unsigned *__restrict__ state)
 {
     pdl_wait();
     pdl_launch_next();
-    const int2 wk = work[blockIdx.x];
-    if (__ldcg(gmask + wk.x) & 1u) return;
+    const int2 wk = work ? work[blockIdx.x] : make_int2(first, (int)blockIdx.x);
+    if (__ldcg(state + wk.x) & kStopped) return;
     const GroupDev &G = groups[wk.x];
     const VolDev &V = vols[G.vol];
     int bx, by, bz;
     decode_tile(V, wk.y, bx, by, bz);
     const int x = bx * kBX + threadIdx.x, y = by * kBY + threadIdx.y;
-#if (M16_BATCH1_SMEM_VIEW & 1)
     // the view in shared memory: its fields are read where used instead of
     // held in registers for the whole column
     __shared__ FlowView sf;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        float *st = (float *)G.state;
+        float *st = G.state;
         const int64_t S = G.slab;
         sf.d0 = V.d0; sf.d1 = V.d1; sf.d2 = V.d2;
         sf.ss0 = V.ss0; sf.ss1 = V.ss1; sf.ss2 = V.ss2;
         sf.sq0 = G.sq0; sf.sq1 = G.sq1; sf.sq2 = G.sq2; sf.isq0 = G.isq0; sf.isq1 = G.isq1; sf.isq2 = G.isq2;
         sf.alpha_scalar = 0.f;
-        sf.alpha = G.alpha1;
+        sf.alpha = G.alpha;
         sf.grad2 = V.grad2;
-        sf.w = G.w.x;
-        sf.neg_inv_decay2 = G.nid2.x;
+        sf.w = G.w;
+        sf.neg_inv_decay2 = G.nid2;
         sf.sqeigs = nullptr;
         sf.q4 = V.q4;
         sf.tmp = st + 4 * S;
@@ -467,42 +442,21 @@ __global__ void __launch_bounds__(kTile, M16_BATCH1_MINB) bt1_flow_kernel(const 
     }
     __syncthreads();
     if (x >= sf.d2 || y >= sf.d1) return;
-    const int zc = V.zc;
-    const int z0 = bz * zc, z1 = min(z0 + zc, sf.d0);
-    flow_column<false, ALPHA, M16_BATCH1_FZB>(sf, x, y, z0, z1);
-#else
-    if (x >= V.d2 || y >= V.d1) return;
-    const int z0 = bz * V.zc, z1 = min(z0 + V.zc, V.d0);
-    float *st = (float *)G.state;
-    const int64_t S = G.slab;
-    FlowView f;
-    f.d0 = V.d0; f.d1 = V.d1; f.d2 = V.d2;
-    f.ss0 = V.ss0; f.ss1 = V.ss1; f.ss2 = V.ss2;
-    f.sq0 = G.sq0; f.sq1 = G.sq1; f.sq2 = G.sq2; f.isq0 = G.isq0; f.isq1 = G.isq1; f.isq2 = G.isq2;
-    f.alpha_scalar = 0.f;
-    f.alpha = G.alpha1;
-    f.grad2 = V.grad2;
-    f.w = G.w.x;
-    f.neg_inv_decay2 = G.nid2.x;
-    f.sqeigs = nullptr;
-    f.q4 = V.q4;
-    f.tmp = st + 4 * S;
-    f.hp0 = st; f.hp1 = st + S; f.hp2 = st + 2 * S;
-    flow_column<false, ALPHA, M16_BATCH1_FZB>(f, x, y, z0, z1);
-#endif
+    const int z0 = bz * V.zc;
+    flow_column<false, ALPHA>(sf, x, y, z0, min(z0 + V.zc, sf.d0));
 }
 
 template <bool CHECK>
-__global__ void __launch_bounds__(kTile, M16_BATCH1_MINB) bt1_label_kernel(const int2 *__restrict__ work,
-                                                                          const VolDev *vols, const GroupDev *groups,
-                                                                          const unsigned *__restrict__ gmask,
-                                                                          float4 *__restrict__ partials)
+__global__ void __launch_bounds__(kTile, CHECK ? 3 : kCompactBlocks) bt1_label_kernel(const int2 *__restrict__ work, int first,
+                                                                         const VolDev *vols, const GroupDev *groups,
+                                                                         const unsigned *__restrict__ state,
+                                                                         float *__restrict__ partials)
 {
     pdl_wait();
     pdl_launch_next();
-    __shared__ float red[kTile / 32];
-    const int2 wk = work[blockIdx.x];
-    if (__ldcg(gmask + wk.x) & 1u) return;   // uniform over the block
+    __shared__ float red[32];
+    const int2 wk = work ? work[blockIdx.x] : make_int2(first, (int)blockIdx.x);
+    if (__ldcg(state + wk.x) & kStopped) return;   // uniform over the block
     const GroupDev &G = groups[wk.x];
     const VolDev &V = vols[G.vol];
     int bx, by, bz;
@@ -510,22 +464,8 @@ __global__ void __launch_bounds__(kTile, M16_BATCH1_MINB) bt1_label_kernel(const
     const int x = bx * kBX + threadIdx.x, y = by * kBY + threadIdx.y;
     const int z0 = bz * V.zc, z1 = min(z0 + V.zc, V.d0);
     float acc = 0.f;
-#if (M16_BATCH1_SMEM_VIEW & 2)
-    __shared__ LabelView sl;   // read where used, not held in registers
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        float *st = (float *)G.state;
-        const int64_t S = G.slab;
-        sl.d0 = V.d0; sl.d1 = V.d1; sl.d2 = V.d2;
-        sl.rcc = V.rcc; sl.rs0 = V.rs0; sl.rs1 = V.rs1; sl.rs2 = V.rs2;
-        sl.hp0 = st; sl.hp1 = st + S; sl.hp2 = st + 2 * S;
-        sl.cs = V.cs; sl.ct = V.ct; sl.labels = nullptr;
-        sl.pt = st + 3 * S; sl.tmp = st + 4 * S; sl.u = st + 5 * S;
-    }
-    __syncthreads();
-    if (x < sl.d2 && y < sl.d1) acc = label_column<false, M16_BATCH1_UZB>(sl, x, y, z0, z1);
-#else
     if (x < V.d2 && y < V.d1) {
-        float *st = (float *)G.state;
+        float *st = G.state;
         const int64_t S = G.slab;
         LabelView l;
         l.d0 = V.d0; l.d1 = V.d1; l.d2 = V.d2;
@@ -533,61 +473,95 @@ __global__ void __launch_bounds__(kTile, M16_BATCH1_MINB) bt1_label_kernel(const
         l.hp0 = st; l.hp1 = st + S; l.hp2 = st + 2 * S;
         l.cs = V.cs; l.ct = V.ct; l.labels = nullptr;
         l.pt = st + 3 * S; l.tmp = st + 4 * S; l.u = st + 5 * S;
-        acc = label_column<false, M16_BATCH1_UZB>(l, x, y, z0, z1);
+        acc = label_column<false>(l, x, y, z0, z1);
     }
-#endif
     if (CHECK) {
-        const int tid = threadIdx.x + kBX * threadIdx.y;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if ((tid & 31) == 0) red[tid >> 5] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            float s = red[0];
-            for (int w = 1; w < kTile / 32; ++w) s += red[w];
-            partials[G.part_off + wk.y] = make_float4(s, 0.f, 0.f, 0.f);
-        }
+        const float s = block_sum(acc, red);
+        if (threadIdx.x == 0 && threadIdx.y == 0) partials[G.part_off + wk.y] = s;
     }
 }
 
-// one block per instance: residual = sum over the tiles of its lane's partial
-// sums / (N * rcc); below the bound (or NaN) the instance stops.  Every
-// instance is checked at its own iterations 0, update, 2 update, ..., so the
-// n-th check (from 0) follows iteration n * update and a stop there counts
-// n * update + 1 iterations, wherever the instance joined the batch.
-__global__ void bt_check_kernel(const VolDev *vols, const GroupDev *groups, const InstDev *insts,
-                                InstCtrl *ctrl, unsigned *gmask, const float4 *__restrict__ partials, double bound,
-                                int update, const int *__restrict__ list)
+inline void compact_volume(VolDev &d, int d0, int d1, int d2, int zc, const TileView &V)
 {
-    pdl_wait();
-    pdl_launch_next();
-    __shared__ double s[256];
-    const int inst = list ? list[blockIdx.x] : (int)blockIdx.x;   // list: the instances to check
-    const InstDev &I = insts[inst];
-    InstCtrl &C = ctrl[inst];
-    if (__ldcg(&C.stopped)) return;
-    const GroupDev &G = groups[I.group];
-    const VolDev &V = vols[G.vol];
-    const float *p = (const float *)(partials + G.part_off) + I.lane;
-    double acc = 0.0;
-    for (int k = threadIdx.x; k < G.nparts; k += blockDim.x) acc += (double)p[4 * k];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x >> 1; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-        __syncthreads();
+    d.d0 = d0; d.d1 = d1; d.d2 = d2;
+    d.zc = zc;
+    d.tx = (int)div_up(d2, kBX); d.ty = (int)div_up(d1, kBY); d.tz = (int)div_up(d0, zc);
+    d.pad = 0;
+    d.rcc = V.rcc; d.rs0 = V.rs0; d.rs1 = V.rs1; d.rs2 = V.rs2; d.ss0 = V.ss0; d.ss1 = V.ss1; d.ss2 = V.ss2;
+}
+
+// z-slices per block of the compact sweeps: four blocks per SM for the volume
+// alone, at least two slices, whole load batches
+inline int compact_zc(int d0, int d1, int d2)
+{
+    const int64_t cols = div_up(d2, kBX) * div_up(d1, kBY);
+    const int64_t zc = (int64_t)d0 * cols / (4 * kSMs);
+    return (int)std::max<int64_t>(std::min<int64_t>(2, d0), std::min<int64_t>(32, zc));
+}
+
+inline int compact_tiles(int d0, int d1, int d2)
+{
+    return (int)(div_up(d2, kBX) * div_up(d1, kBY) * div_up(d0, compact_zc(d0, d1, d2)));
+}
+
+// ---- launches --------------------------------------------------------------------
+
+// the device tables and the work list of a batch or a server step
+struct BatchTables {
+    const int2 *work = nullptr;
+    int first = 0;               // work == NULL: tiles of this instance
+    int seg[kKinds + 1] = {};    // items seg[k] .. seg[k + 1] - 1 are of kind k
+    const TileDev *tiles = nullptr;
+    const VolDev *vols = nullptr;
+    const GroupDev *groups = nullptr;
+    const InstDev *insts = nullptr;
+    InstCtrl *ctrl = nullptr;
+    unsigned *state = nullptr;
+    float *partials = nullptr;
+};
+
+// Enqueues m iterations of the work items; `check` computes the residual sums
+// of the last one (the caller launches the check).  e: optional events around
+// each launch.  Returns the number of sweep launches of the tile kinds (their
+// buffers alternated that often) or -1 on a launch error.
+inline int enqueue_iterations(const BatchTables &T, int m, bool check, cudaStream_t st, int &launches)
+{
+    cudaError_t e = cudaSuccess;
+    auto keep = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    int done = 0, sweeps = 0;
+    while (done < m) {
+        const int k = (m - done) & 1 ? 1 : 2;
+        const bool last = done + k == m;
+        for (int kind = 0; kind < kTileKinds; ++kind) {
+            const int items = T.seg[kind + 1] - T.seg[kind];
+            if (items <= 0) continue;
+            const BatchTileLaunch L = batch_tile_pick(kind, k, check && last);
+            keep(launch_pdl_smem(L.kernel, dim3(items), dim3(kTileLanes, kTileNW), L.smem, st, true,
+                                 T.work ? T.work + T.seg[kind] : nullptr, T.first, T.tiles,
+                                 (const unsigned *)T.state, T.partials, sweeps & 1));
+            ++launches;
+        }
+        done += k;
+        ++sweeps;
     }
-    if (threadIdx.x == 0) {
-        const double err = s[0] / ((double)V.n * (double)V.rcc);
-        C.resid = err;
-        const int n = C.n_checks;
-        C.n_checks = n + 1;
-        if (isnan(err) || err < bound) {
-            C.stopped = 1;
-            C.iterations = n * update + 1;
-            atomicOr(gmask + I.group, 1u << I.lane);
+    const int na = T.seg[kCompactAlpha + 1] - T.seg[kCompactAlpha];
+    const int ne = T.seg[kCompactExp + 1] - T.seg[kCompactExp];
+    if (na + ne > 0) {
+        const dim3 block(kBX, kBY, 1);
+        const int2 *wa = T.work ? T.work + T.seg[kCompactAlpha] : nullptr;
+        const int2 *we = T.work ? T.work + T.seg[kCompactExp] : nullptr;
+        const unsigned *state = T.state;
+        for (int i = 0; i < m; ++i) {
+            if (na > 0) keep(launch_pdl(bt1_flow_kernel<kAlphaArray>, dim3(na), block, st, true, wa, T.first, T.vols, T.groups, state));
+            if (ne > 0) keep(launch_pdl(bt1_flow_kernel<kAlphaFromGrad2>, dim3(ne), block, st, true, we, T.first, T.vols, T.groups, state));
+            if (check && i == m - 1)
+                keep(launch_pdl(bt1_label_kernel<true>, dim3(na + ne), block, st, true, wa, T.first, T.vols, T.groups, state, T.partials));
+            else
+                keep(launch_pdl(bt1_label_kernel<false>, dim3(na + ne), block, st, true, wa, T.first, T.vols, T.groups, state, T.partials));
+            launches += (na > 0) + (ne > 0) + 1;
         }
     }
+    return e == cudaSuccess ? sweeps : -1;
 }
 
 }  // namespace

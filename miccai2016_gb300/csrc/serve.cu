@@ -1,14 +1,15 @@
 // serve.cu -- continuous batching of ATV max-flow requests (m16_server_*).
 //
-// A request is one volume with its own solve (a one-lane group of the batched
+// A request is one volume with its own solve (an instance of the batched
 // engine, batch_kernels.cuh).  The server holds one caller workspace: its
 // tables (descriptors, control words, work list) at the front and an arena for
 // the requests behind them.  Admission allocates a request's inputs, state and
 // partial sums in one arena block; the inputs are uploaded on the server's copy
 // stream and the set-up kernels run on the compute stream behind an event, so
-// uploads overlap the iterations of resident requests.  A step runs
-// params->update iterations of every resident request (one residual check, at
-// the first), reads the stop mask, retires requests at the bound or at
+// uploads overlap the iterations of resident requests; iteration 0 and its
+// check follow the set-up.  A step runs the params->update iterations up to the
+// next check of every resident request (without a check for a request in its
+// last iterations), reads the stop mask, retires requests at the bound or at
 // num_iter, and starts their u downloads on the copy stream; poll() hands out
 // requests whose download has finished and returns their memory.
 //
@@ -24,6 +25,7 @@
 #include <algorithm>
 #include <iterator>
 #include <map>
+#include <utility>
 #include <vector>
 
 #include "batch_kernels.cuh"
@@ -32,7 +34,6 @@ namespace m16 {
 namespace {
 
 constexpr size_t kAlign = 256;
-constexpr int kSetupBlocks = 4 * kSMs;
 
 // first-fit allocator over [0, size) in 256-byte granules; adjacent free
 // ranges are merged on release
@@ -91,56 +92,69 @@ private:
     std::map<size_t, size_t> free_, used_;   // offset -> size
 };
 
-// z-chunk of a request's tiles: about M16_SERVE_BLOCKS_PER_SM blocks per SM
-// for the request alone, at least two slices (the sweeps load two slices at a
-// time)
-#ifndef M16_SERVE_BLOCKS_PER_SM
-#define M16_SERVE_BLOCKS_PER_SM 4
-#endif
-#ifndef M16_SERVE_MIN_ZC
-#define M16_SERVE_MIN_ZC 2
-#endif
-inline int serve_zc(int d0, int d1, int d2)
-{
-    const int64_t cols = div_up(d2, kBX) * div_up(d1, kBY);
-    const int64_t zc = (int64_t)d0 * cols / (M16_SERVE_BLOCKS_PER_SM * kSMs);
-    return (int)std::max<int64_t>(std::min<int64_t>(M16_SERVE_MIN_ZC, d0), std::min<int64_t>(32, zc));
-}
-
-// where a request's fields sit in its arena block
+// Where a request's fields sit in its arena block.  Tile sweeps: 72 bytes a
+// voxel, the two state buffers, the directions and the capacities.  The inputs
+// are read by the set-up kernels only and share that memory: the image sits
+// where the capacities go (the state is written first), the others where the
+// second state buffer is, the maximum where the directions go; the result is
+// gathered there at the end.  Compact: the inputs stay, one planar state.
 struct ReqLayout {
-    size_t img, quat3, alpha, cs, ct, q4, state, partials, maxpart, total;
-    int zc, tx, ty, tz;
+    size_t img, quat3, alpha, cs, ct, maxpart, denom, total;
+    size_t h[2], u[2], dir, caps, rad;         // tile sweeps
+    size_t q4, state;                          // compact sweeps
+    size_t partials;                           // tiles > kSlotPartials
+    int tiles, zc;
+    bool compact;
     int64_t n, slab;
 };
 
-inline ReqLayout req_layout(int d0, int d1, int d2)
+constexpr int kSlotPartials = 1024;   // partial sums kept in the server's tables per slot
+
+inline ReqLayout req_layout(int d0, int d1, int d2, bool compact, bool rad)
 {
     ReqLayout R;
     const int64_t n = (int64_t)d0 * d1 * d2;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, kAlign); return o; };
     R.n = n;
-    R.img = take(n * 4);
+    R.compact = compact;
     R.quat3 = take(n * 12);
     R.alpha = take(n * 4);   // |grad I|^2, or the per-voxel alpha
     R.cs = take(n * 4);
     R.ct = take(n * 4);
-    R.q4 = take(n * 16);
     R.slab = (int64_t)(align_up(n * 4, kAlign) / 4);
-    R.state = take(kFields * R.slab * 4);
-    R.zc = serve_zc(d0, d1, d2);
-    R.tx = (int)div_up(d2, kBX);
-    R.ty = (int)div_up(d1, kBY);
-    R.tz = (int)div_up(d0, R.zc);
-    R.partials = take((size_t)R.tx * R.ty * R.tz * 16);
-    R.maxpart = take(kSetupBlocks * 4);
+    if (compact) {
+        R.img = take(n * 4);
+        R.q4 = take(n * 16);
+        R.state = take(kFields * R.slab * 4);
+        R.zc = compact_zc(d0, d1, d2);
+        R.tiles = compact_tiles(d0, d1, d2);
+        R.maxpart = take(kSetupBlocks * 4);
+        R.denom = take(4);
+    } else {
+        const size_t np = (size_t)tile_voxels(d0, d1, d2);
+        R.h[1] = 0;
+        R.u[1] = align_up(np * 16, kAlign);
+        off = std::max(off, R.u[1] + align_up(np * 8, kAlign));
+        R.h[0] = take(np * 16);
+        R.u[0] = take(np * 8);
+        R.dir = take(std::max<size_t>(np * 16, kSetupBlocks * 4 + 4));
+        R.caps = R.img = take(np * 8);
+        R.rad = rad ? take(np * 4) : 0;
+        R.maxpart = R.dir;
+        R.denom = R.dir + kSetupBlocks * 4;
+        // the chunk of z as if four such requests shared the device
+        const int nx = tile_count_x(d2), ny = tile_count_y(d1, kTileRows);
+        R.zc = tile_zc(d0, 4 * (int64_t)nx * ny);
+        R.tiles = (int)(nx * ny * div_up(d0, R.zc));
+    }
+    R.partials = R.tiles > kSlotPartials ? take((size_t)R.tiles * 4) : 0;
     R.total = off;
     return R;
 }
 
 struct Tables {
-    size_t vols, groups, insts, ctrl, gmask, work, list, total;
+    size_t vols, tiles, maps, groups, insts, ctrl, state, work, list, partials, err, total;
 };
 
 inline Tables tables(int max_slots, int max_work)
@@ -149,12 +163,16 @@ inline Tables tables(int max_slots, int max_work)
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, kAlign); return o; };
     T.vols = take(sizeof(VolDev) * max_slots);
+    T.tiles = take(sizeof(TileDev) * max_slots);
+    T.maps = take(8 * sizeof(CUtensorMap) * max_slots);
     T.groups = take(sizeof(GroupDev) * max_slots);
     T.insts = take(sizeof(InstDev) * max_slots);
     T.ctrl = take(sizeof(InstCtrl) * max_slots);
-    T.gmask = take(sizeof(unsigned) * max_slots);
+    T.state = take(sizeof(unsigned) * max_slots);
     T.work = take(sizeof(int2) * (size_t)max_work);
     T.list = take(sizeof(int) * max_slots);
+    T.partials = take(sizeof(float) * kSlotPartials * (size_t)max_slots);
+    T.err = take(sizeof(int));
     T.total = off;
     return T;
 }
@@ -163,14 +181,14 @@ enum SlotState { kFree = 0, kResident = 1, kDraining = 2 };
 
 struct Slot {
     int state = kFree;
-    int iters_planned = 0;   // iterations of the steps enqueued so far (before any stop is known)
+    int iters_planned = 0;   // iterations enqueued so far (before any stop is known)
+    bool done_planning = false;   // its last step is enqueued
     int64_t last_listed = -1;   // the last step whose work list holds the slot
     int64_t tag = 0;
     size_t block = 0;        // arena offset (from the arena's base)
-    size_t u_off = 0;        // workspace offset of u
+    size_t u_off = 0;        // workspace offset of the contiguous u
     int64_t n = 0;
-    int tiles = 0;
-    bool alpha = false;
+    int tiles = 0, kind = 0;
     int iters_done = 0;      // iterations run so far
     int iterations = 0;      // at retirement
     double resid = NAN;
@@ -181,10 +199,12 @@ struct Slot {
 // pinned host copies of one slot's descriptors, uploaded at admission
 struct Staging {
     VolDev vol;
+    TileDev tile;
     GroupDev group;
     InstDev inst;
     InstCtrl ctrl;
-    unsigned mask;
+    unsigned state;
+    CUtensorMap maps[8];
 };
 
 }  // namespace
@@ -212,13 +232,17 @@ struct m16_server {
     Staging *stage = nullptr;        // max_slots
     int2 *work_h[2] = {nullptr, nullptr};   // max_work each, by rebuild parity
     int *list_h[2] = {nullptr, nullptr};    // max_slots each, by rebuild parity
-    unsigned *mask_h = nullptr;      // max_slots
     InstCtrl *ctrl_h[2] = {nullptr, nullptr};   // max_slots each, by step parity
-    int seg_alpha = 0, n_items = 0;  // work items: [0, seg_alpha) alpha fields, [seg_alpha, n_items) (w, decay)
-    int n_list = 0;                  // slots in the current list
+    int *err_h = nullptr;            // by step parity: a sweep's copies did not arrive
+    // the work list: requests whose step ends with a check, then those in
+    // their last iterations; the check list holds the former first
+    int seg[2][kKinds + 1] = {};
+    int n_full = 0, n_list = 0;      // slots with a check, slots in the current list
     int64_t rebuilds = 0;
     std::vector<int> list_cur;       // the current list (host copy)
-    std::vector<int> step_list[2];   // the list of each step in flight, by step parity
+    // the list of each step in flight, by step parity: slots and the
+    // iterations they have run after it
+    std::vector<std::pair<int, int>> step_list[2];
     int64_t steps = 0;               // steps enqueued
     int64_t processed = 0;           // steps whose stop masks have been read (all steps < processed)
     int64_t voxel_iterations = 0;    // iterations that ran, times each request's voxels
@@ -245,14 +269,22 @@ void release_host(m16_server *s)
         if (s->t_start[b]) cudaEventDestroy(s->t_start[b]);
         if (s->t_end[b]) cudaEventDestroy(s->t_end[b]);
     }
-    if (s->mask_h) cudaFreeHost(s->mask_h);
+    if (s->err_h) cudaFreeHost(s->err_h);
     for (Slot &sl : s->slots)
         if (sl.ev) cudaEventDestroy(sl.ev);
     if (s->copy) cudaStreamDestroy(s->copy);
 }
 
+// whether the slot's next step ends with a check: iteration 0 and its check ran
+// at admission, a step is the `update` iterations up to the next check, the
+// last step those that remain without one
+bool full_step(const m16_server *s, const Slot &sl)
+{
+    return sl.iters_planned - 1 + s->params.update < s->params.num_iter;
+}
+
 // rebuild the work list and the check list over the resident slots that
-// still have iterations to run.  The host sources alternate by rebuild: the
+// still have a step to run.  The host sources alternate by rebuild: the
 // copy from a buffer is ordered before the step enqueued after it, which has
 // been processed (its stop mask read) before the buffer's next rebuild.
 int rebuild(m16_server *s)
@@ -263,18 +295,21 @@ int rebuild(m16_server *s)
     int nw = 0, nl = 0;
     s->list_cur.clear();
     for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1) s->seg_alpha = nw;
-        for (int k = 0; k < s->max_slots; ++k) {
-            const Slot &sl = s->slots[k];
-            if (sl.state != kResident || sl.alpha != (pass == 0)) continue;
-            if (sl.iters_planned >= s->params.num_iter) continue;   // its last step is enqueued
-            if (nw + sl.tiles > s->max_work) return M16_ERR_TOO_LARGE;
-            for (int t = 0; t < sl.tiles; ++t) work[nw++] = make_int2(k, t);
-            list[nl++] = k;
-            s->list_cur.push_back(k);
+        for (int kind = 0; kind < kKinds; ++kind) {
+            s->seg[pass][kind] = nw;
+            for (int k = 0; k < s->max_slots; ++k) {
+                const Slot &sl = s->slots[k];
+                if (sl.state != kResident || sl.kind != kind || sl.done_planning) continue;
+                if (full_step(s, sl) != (pass == 0)) continue;
+                if (nw + sl.tiles > s->max_work) return M16_ERR_TOO_LARGE;
+                for (int t = 0; t < sl.tiles; ++t) work[nw++] = make_int2(k, t);
+                list[nl++] = k;
+                s->list_cur.push_back(k);
+            }
         }
+        s->seg[pass][kKinds] = nw;
+        if (pass == 0) s->n_full = nl;
     }
-    s->n_items = nw;
     s->n_list = nl;
     if (nw > 0)
         M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.work, work, sizeof(int2) * nw, cudaMemcpyHostToDevice, s->stream));
@@ -285,13 +320,42 @@ int rebuild(m16_server *s)
     return M16_OK;
 }
 
+BatchTables server_tables(m16_server *s)
+{
+    BatchTables B;
+    B.work = (const int2 *)(s->ws + s->T.work);
+    B.tiles = (const TileDev *)(s->ws + s->T.tiles);
+    B.vols = (const VolDev *)(s->ws + s->T.vols);
+    B.groups = (const GroupDev *)(s->ws + s->T.groups);
+    B.insts = (const InstDev *)(s->ws + s->T.insts);
+    B.ctrl = (InstCtrl *)(s->ws + s->T.ctrl);
+    B.state = (unsigned *)(s->ws + s->T.state);
+    B.partials = (float *)s->ws;   // part_off counts floats from the workspace start
+    return B;
+}
+
+cudaError_t launch_check(m16_server *s, const BatchTables &B, int count, const int *list, int first, int flip)
+{
+    return launch_pdl(bt_check_kernel, dim3(count), dim3(256), s->stream, true, B.insts, B.ctrl, B.state,
+                      (const float *)B.partials, s->params.error_bound, s->params.update, flip, list, first);
+}
+
 // the retired slot's u goes to the host on the copy stream, after the step
-// (of parity b) in which it became final
-int start_download(m16_server *s, int k, int b)
+// (of parity b) in which it became final; flip: that step ended without the
+// check that stores the current buffer, after an odd number of launches
+int start_download(m16_server *s, int k, int b, int flip)
 {
     Slot &sl = s->slots[k];
     sl.state = kDraining;
     M16_CUDA_TRY(cudaStreamWaitEvent(s->copy, s->step_end[b], 0));
+    if (sl.kind < kTileKinds) {
+        // the tile sweeps' u is padded and beside p_t: gathered first (steps
+        // that still list the slot do not touch it any more)
+        const int blocks = (int)std::min<int64_t>(kSetupBlocks, div_up(sl.n, 256));
+        const BatchTables B = server_tables(s);
+        bt_result_kernel<<<dim3(blocks, 1), 256, 0, s->copy>>>(B.insts, B.state, k, flip);
+        M16_CUDA_TRY(cudaGetLastError());
+    }
     M16_CUDA_TRY(cudaMemcpyAsync(sl.u_host, s->ws + sl.u_off, sl.n * 4, cudaMemcpyDeviceToHost, s->copy));
     M16_CUDA_TRY(cudaEventRecord(sl.ev, s->copy));
     s->dirty = true;
@@ -325,7 +389,7 @@ extern "C" size_t m16_server_request_bytes(int32_t d0, int32_t d1, int32_t d2, i
 {
     (void)has_alpha;   // the alpha field takes the place of |grad I|^2
     if (d0 < 1 || d1 < 1 || d2 < 1 || (int64_t)d0 * d1 * d2 > (int64_t)INT32_MAX) return 0;
-    return req_layout(d0, d1, d2).total;
+    return req_layout(d0, d1, d2, !tile_shape_ok(d0, d1, d2), false).total;
 }
 
 extern "C" size_t m16_server_table_bytes(int32_t max_slots, int32_t max_work_items)
@@ -359,7 +423,9 @@ extern "C" int m16_server_create(const m16_cut_params *params, int32_t max_slots
     for (int k = max_slots - 1; k >= 0; --k) s->free_slots.push_back(k);
     bool ok = cudaStreamCreateWithFlags(&s->copy, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMallocHost((void **)&s->stage, sizeof(Staging) * max_slots) == cudaSuccess &&
-              cudaMallocHost((void **)&s->mask_h, sizeof(unsigned) * max_slots) == cudaSuccess;
+              cudaMallocHost((void **)&s->err_h, 2 * sizeof(int)) == cudaSuccess &&
+              cudaMemsetAsync(s->ws + T.err, 0, sizeof(int), s->stream) == cudaSuccess;
+    for (int k = 0; ok && k < kTileKinds; ++k) ok = batch_tile_prepare(k) == cudaSuccess;
     for (int b = 0; ok && b < 2; ++b)
         ok = cudaEventCreateWithFlags(&s->step_end[b], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&s->ctrl_ev[b], cudaEventDisableTiming) == cudaSuccess &&
@@ -390,10 +456,23 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
         if (!(req->scaling[k] > 0.0) || !(req->sqevals[k] > 0.0)) return M16_ERR_BAD_ARG;
     collect(s);
     if (s->free_slots.empty()) return M16_OK;
-    const ReqLayout R = req_layout(req->d0, req->d1, req->d2);
-    if (R.tx * R.ty * R.tz > s->max_work) return M16_ERR_TOO_LARGE;
+    TileView view = TileView();
+    int axis;
+    const int metric = tile_metric(req->sqevals, view, &axis);
+    tile_view(view, req->d0, req->d1, req->d2, req->scaling, s->params);
+    const bool rad = metric == kMetricConst;   // a radius field beside the quaternions
+    ReqLayout R = req_layout(req->d0, req->d1, req->d2, !tile_shape_ok(req->d0, req->d1, req->d2), rad);
     size_t block;
-    if (!s->arena.alloc(R.total, &block)) return M16_OK;
+    if (R.tiles > s->max_work || !s->arena.alloc(R.total, &block)) {
+        // A request that the tile sweeps' fields do not fit even alone takes the
+        // compact sweeps' (68 bytes a voxel); others wait for room.
+        const bool alone = (int)s->free_slots.size() == s->max_slots;
+        const ReqLayout C = req_layout(req->d0, req->d1, req->d2, true, false);
+        if (R.tiles > s->max_work && C.tiles > s->max_work) return M16_ERR_TOO_LARGE;
+        if ((R.tiles <= s->max_work && !alone) || C.tiles > s->max_work || !s->arena.alloc(C.total, &block))
+            return M16_OK;
+        R = C;
+    }
     const int k = s->free_slots.back();
     s->free_slots.pop_back();
     Slot &sl = s->slots[k];
@@ -411,81 +490,139 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
 
     // descriptors (staged in pinned memory, uploaded on the copy stream too)
     Staging &S = s->stage[k];
-    VolDev &v = S.vol;
-    const double *sc = req->scaling;
-    const double smin = fmin(sc[0], fmin(sc[1], sc[2]));
-    const m16_cut_params &p = s->params;
-    v.d0 = req->d0; v.d1 = req->d1; v.d2 = req->d2;
-    v.zc = R.zc; v.tx = R.tx; v.ty = R.ty; v.tz = R.tz; v.pad = 0;
-    v.rcc = (float)(1.0 / (p.cc * (smin * smin)));
-    v.rs0 = (float)(1.0 / sc[0]); v.rs1 = (float)(1.0 / sc[1]); v.rs2 = (float)(1.0 / sc[2]);
-    v.ss0 = (float)(p.steps / sc[0] * (smin * smin));
-    v.ss1 = (float)(p.steps / sc[1] * (smin * smin));
-    v.ss2 = (float)(p.steps / sc[2] * (smin * smin));
-    v.denom = 1.f;
-    v.q4 = (const float4 *)(base + R.q4);
-    v.grad2 = req->alpha ? nullptr : (const float *)(base + R.alpha);
-    v.cs = (const float *)(base + R.cs);
-    v.ct = (const float *)(base + R.ct);
-    v.n = n;
-    GroupDev &g = S.group;
-    g.part_off = (int64_t)((s->arena_base + block + R.partials) / 16);
-    g.vol = k;
-    g.nparts = R.tx * R.ty * R.tz;
-    g.has_alpha = req->alpha ? 1 : 0;
-    g.lanes = 1;
-    g.pad0 = g.pad1 = g.pad2 = 0;
-    g.w = make_float4((float)req->weighting, 0.f, 0.f, 0.f);
-    g.nid2 = make_float4(req->alpha ? 0.f : (float)(-1.0 / (req->decay * req->decay)), 0.f, 0.f, 0.f);
-    g.sq0 = (float)req->sqevals[0]; g.sq1 = (float)req->sqevals[1]; g.sq2 = (float)req->sqevals[2];
-    g.isq0 = (float)(1.0 / req->sqevals[0]); g.isq1 = (float)(1.0 / req->sqevals[1]);
-    g.isq2 = (float)(1.0 / req->sqevals[2]);
-    g.state = base + R.state;
-    g.slab = R.slab;
-    g.alpha1 = req->alpha ? (const float *)(base + R.alpha) : nullptr;
-    S.inst.group = k;
-    S.inst.lane = 0;
+    const float *img = (const float *)(base + R.img), *quat3 = (const float *)(base + R.quat3);
+    const float *value = (const float *)(base + R.alpha), *cs = (const float *)(base + R.cs),
+                *ct = (const float *)(base + R.ct);
+    float *denom = (float *)(base + R.denom);
+    const float w = (float)req->weighting;
+    const float nid2 = req->alpha ? 0.f : (float)(-1.0 / (req->decay * req->decay));
+    const int64_t part_off = (int64_t)((R.tiles > kSlotPartials ? s->arena_base + block + R.partials
+                                                                 : s->T.partials + sizeof(float) * kSlotPartials * k) / 4);
+    S.inst.n = n;
+    S.inst.part_off = part_off;
+    S.inst.nparts = R.tiles;
+    S.inst.d2 = req->d2;
+    S.inst.rcc = view.rcc;
+    S.inst.u2[0] = S.inst.u2[1] = nullptr;
+    S.inst.u1 = nullptr;
     S.inst.u_out = nullptr;
-    S.inst.alpha = g.alpha1;
-    S.ctrl.stopped = 0;
-    S.ctrl.iterations = p.num_iter;
-    S.ctrl.n_checks = 0;
-    S.ctrl.pad = 0;
-    S.ctrl.resid = NAN;
-    S.mask = kAllLanes & ~1u;   // lanes 1..3 do not exist
-    M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.vols + sizeof(VolDev) * k, &S.vol, sizeof(VolDev),
-                                 cudaMemcpyHostToDevice, cp));
-    M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.groups + sizeof(GroupDev) * k, &S.group, sizeof(GroupDev),
-                                 cudaMemcpyHostToDevice, cp));
-    M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.insts + sizeof(InstDev) * k, &S.inst, sizeof(InstDev),
-                                 cudaMemcpyHostToDevice, cp));
-    M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.ctrl + sizeof(InstCtrl) * k, &S.ctrl, sizeof(InstCtrl),
-                                 cudaMemcpyHostToDevice, cp));
-    M16_CUDA_TRY(cudaMemcpyAsync(s->ws + s->T.gmask + sizeof(unsigned) * k, &S.mask, sizeof(unsigned),
-                                 cudaMemcpyHostToDevice, cp));
+    S.vol = VolDev();
+    S.group = GroupDev();
+    S.tile = TileDev();
+    VolumeFields F = VolumeFields();
+    if (R.compact) {
+        compact_volume(S.vol, req->d0, req->d1, req->d2, R.zc, view);
+        S.vol.q4 = (const float4 *)(base + R.q4);
+        S.vol.grad2 = req->alpha ? nullptr : value;
+        S.vol.cs = cs; S.vol.ct = ct;
+        GroupDev &g = S.group;
+        g.vol = k;
+        g.part_off = part_off;
+        g.w = w;
+        g.nid2 = nid2;
+        g.sq0 = view.sq0; g.sq1 = view.sq1; g.sq2 = view.sq2;
+        g.isq0 = view.isq0; g.isq1 = view.isq1; g.isq2 = view.isq2;
+        g.state = (float *)(base + R.state);
+        g.slab = R.slab;
+        g.alpha = req->alpha ? value : nullptr;
+        g.img = img;
+        g.denom = denom;
+        S.inst.u1 = g.state + 5 * g.slab;
+        sl.kind = req->alpha ? kCompactAlpha : kCompactExp;
+    } else {
+        TileDev &t = S.tile;
+        t.V = view;
+        t.V.exp_radius = req->alpha ? 0 : 1;
+        t.V.w = w;
+        t.V.nid2 = nid2;
+        t.V.labels = nullptr;
+        t.V.err = (int *)(s->ws + s->T.err);
+        CUtensorMap *dm = (CUtensorMap *)(s->ws + s->T.maps) + 8 * k;
+        bool ok = true;
+        for (int b = 0; b < 2; ++b) {
+            t.h[b] = (float4 *)(base + R.h[b]);
+            t.u[b] = (float2 *)(base + R.u[b]);
+            ok = ok && tile_map(S.maps + b, t.h[b], req->d0, req->d1, view.pitch, 4, kTileRows + 1) &&
+                 tile_map(S.maps + 2 + b, t.u[b], req->d0, req->d1, view.pitch, 2, kTileRows);
+            t.mh[b] = dm + b;
+            t.mu[b] = dm + 2 + b;
+            S.inst.u2[b] = t.u[b];
+        }
+        F.caps = (float2 *)(base + R.caps);
+        ok = ok && tile_map(S.maps + 4, F.caps, req->d0, req->d1, view.pitch, 2, kTileRows);
+        t.V.mcaps = dm + 4;
+        // the direction with the radius, the radius alone in its place, or the
+        // quaternion and a radius field
+        if (metric == kMetricAxis) F.dir[axis] = (float4 *)(base + R.dir);
+        else if (metric == kMetricConst) F.q4 = (float4 *)(base + R.dir);
+        if (metric != kMetricAxis) F.rad = (float *)(base + (metric == kMetricConst ? R.rad : R.dir));
+        if (metric != kMetricIso)
+            ok = ok && tile_map(S.maps + 5, base + R.dir, req->d0, req->d1, view.pitch, 4, kTileRows);
+        if (F.rad) ok = ok && tile_map(S.maps + 6, F.rad, req->d0, req->d1, view.pitch, 1, kTileRows);
+        if (!ok) {
+            s->arena.release(block);
+            s->free_slots.push_back(k);
+            return M16_ERR_CUDA;
+        }
+        t.V.mdir = dm + 5;
+        t.V.mrad = dm + 6;
+        t.part_off = part_off;
+        t.rows = (int64_t)req->d0 * req->d1;
+        t.nx = tile_count_x(req->d2);
+        t.ny = tile_count_y(req->d1, kTileRows);
+        t.zc = R.zc;
+        t.img = img; t.cs = cs; t.ct = ct; t.alpha = nullptr; t.denom = denom; t.rad = nullptr;
+        S.inst.u_out = (float *)(base + R.dir);
+        sl.kind = metric == kMetricAxis ? kAxisPacked : metric == kMetricIso ? kIsoPlanar : kConstPlanar;
+        M16_CUDA_TRY(cudaMemcpyAsync(dm, S.maps, sizeof(S.maps), cudaMemcpyHostToDevice, cp));
+    }
+    S.ctrl = InstCtrl{0, s->params.num_iter, 0, 0, NAN};
+    S.state = 0u;
+    auto up = [&](size_t table, const void *src, size_t bytes) {
+        return cudaMemcpyAsync(s->ws + table + bytes * k, src, bytes, cudaMemcpyHostToDevice, cp);
+    };
+    M16_CUDA_TRY(up(s->T.vols, &S.vol, sizeof(VolDev)));
+    M16_CUDA_TRY(up(s->T.tiles, &S.tile, sizeof(TileDev)));
+    M16_CUDA_TRY(up(s->T.groups, &S.group, sizeof(GroupDev)));
+    M16_CUDA_TRY(up(s->T.insts, &S.inst, sizeof(InstDev)));
+    M16_CUDA_TRY(up(s->T.ctrl, &S.ctrl, sizeof(InstCtrl)));
+    M16_CUDA_TRY(up(s->T.state, &S.state, sizeof(unsigned)));
     M16_CUDA_TRY(cudaEventRecord(sl.ev, cp));
 
-    // set-up on the compute stream once the uploads are in
+    // set-up on the compute stream once the uploads are in, then iteration 0
+    // and its check
     M16_CUDA_TRY(cudaStreamWaitEvent(st, sl.ev, 0));
-    VolDev *dvols = (VolDev *)(s->ws + s->T.vols);
-    const GroupDev *dgroups = (const GroupDev *)(s->ws + s->T.groups);
+    BatchTables B = server_tables(s);
     const int blocks = (int)std::min<int64_t>(kSetupBlocks, div_up(n, 256));
     float *mp = (float *)(base + R.maxpart);
-    bt_max_kernel<<<blocks, 256, 0, st>>>((const float *)(base + R.img), n, mp);
-    bt_denom_kernel<<<1, 32, 0, st>>>(mp, blocks, dvols + k);
-    bt_expand_kernel<<<blocks, 256, 0, st>>>((const float *)(base + R.quat3), (float4 *)(base + R.q4), n);
-    bt_init_group_kernel<<<blocks, 256, 0, st>>>((const float *)(base + R.img), dvols, dgroups, k);
+    bt_max_kernel<<<blocks, 256, 0, st>>>(img, n, mp);
+    bt_denom_kernel<<<1, 256, 0, st>>>(mp, blocks, denom);
+    if (R.compact) {
+        bt_expand_kernel<<<blocks, 256, 0, st>>>(quat3, (float4 *)(base + R.q4), n);
+        bt1_state_kernel<<<dim3(blocks, 1), 256, 0, st>>>(B.vols, B.groups, k);
+    } else {
+        // in this order: the volume's fields overwrite the image and the maximum
+        bt_state_kernel<<<dim3(blocks, 1), 256, 0, st>>>(B.tiles, k);
+        bt_volume_kernel<<<blocks, 256, 0, st>>>(quat3, value, cs, ct, req->d2, (int64_t)req->d0 * req->d1, F);
+    }
     M16_CUDA_TRY(cudaGetLastError());
+    B.work = nullptr;
+    B.first = k;
+    for (int i = sl.kind + 1; i <= kKinds; ++i) B.seg[i] = R.tiles;
+    int launches = 0;
+    const int sweeps = enqueue_iterations(B, 1, true, st, launches);
+    if (sweeps < 0) return M16_ERR_CUDA;
+    M16_CUDA_TRY(launch_check(s, B, 1, nullptr, k, sweeps & 1));
 
     sl.state = kResident;
     sl.tag = req->tag;
     sl.block = block;
-    sl.u_off = s->arena_base + block + R.state + (size_t)5 * R.slab * 4;
+    sl.u_off = s->arena_base + block + (R.compact ? R.state + (size_t)5 * R.slab * 4 : R.dir);
     sl.n = n;
-    sl.tiles = R.tx * R.ty * R.tz;
-    sl.alpha = req->alpha != nullptr;
+    sl.tiles = R.tiles;
     sl.iters_done = 0;
-    sl.iters_planned = 0;
+    sl.iters_planned = 1;
+    sl.done_planning = false;
     sl.last_listed = -1;
     sl.iterations = 0;
     sl.resid = NAN;
@@ -507,21 +644,22 @@ int process_step(m16_server *s, int64_t idx)
     float step_ms = 0.f;
     M16_CUDA_TRY(cudaEventElapsedTime(&step_ms, s->t_start[b], s->t_end[b]));
     s->gpu_ms += step_ms;
-    for (int k : s->step_list[b]) {
+    if (s->err_h[b]) return M16_ERR_TIMEOUT;
+    for (const auto &entry : s->step_list[b]) {
+        const int k = entry.first, target = entry.second;
         Slot &sl = s->slots[k];
         if (sl.state != kResident) continue;   // retired after an earlier step: masked here
         const InstCtrl &c = s->ctrl_h[b][k];
         sl.resid = c.resid;
-        // a request that stopped at this step's check ran that one iteration
-        s->voxel_iterations += sl.n * (c.stopped ? std::max(0, c.iterations - sl.iters_done) : s->params.update);
-        if (c.stopped) {
-            sl.iterations = c.iterations;
-        } else {
-            sl.iters_done += s->params.update;
-            if (sl.iters_done < s->params.num_iter) continue;
-            sl.iterations = s->params.num_iter;
-        }
-        const int r = start_download(s, k, b);
+        // a request that stopped at this step's check (or at iteration 0's)
+        // ran up to it
+        const int ran = c.stopped ? c.iterations : target;
+        s->voxel_iterations += sl.n * std::max(0, ran - sl.iters_done);
+        sl.iters_done = ran;
+        if (!c.stopped && ran < s->params.num_iter) continue;
+        sl.iterations = c.stopped ? c.iterations : s->params.num_iter;
+        // the last iterations end without a check: update / 2 launches
+        const int r = start_download(s, k, b, !c.stopped && (s->params.update / 2) & 1);
         if (r != M16_OK) return r;
     }
     s->processed = idx + 1;
@@ -543,47 +681,36 @@ extern "C" int m16_server_step(m16_server *s)
         cudaStream_t st = s->stream;
         const int64_t c = s->steps;
         const int b = (int)(c & 1);   // step c - 2 of this parity has been processed
-        const VolDev *dvols = (const VolDev *)(s->ws + s->T.vols);
-        const GroupDev *dgroups = (const GroupDev *)(s->ws + s->T.groups);
-        const InstDev *dinsts = (const InstDev *)(s->ws + s->T.insts);
-        InstCtrl *dctrl = (InstCtrl *)(s->ws + s->T.ctrl);
-        unsigned *dmask = (unsigned *)(s->ws + s->T.gmask);
-        const int2 *dwork = (const int2 *)(s->ws + s->T.work);
-        const int *dlist = (const int *)(s->ws + s->T.list);
-        float4 *dpart = (float4 *)s->ws;   // part_off counts float4 from the workspace start
-        const dim3 block(kBX, kBY, 1);
-        const int na = s->seg_alpha, ne = s->n_items - s->seg_alpha;
+        BatchTables B = server_tables(s);
         M16_CUDA_TRY(cudaEventRecord(s->t_start[b], st));
         // programmatic dependent launch between the sweeps (common.cuh); the
         // first sweep follows an event record and launches in stream order
-        for (int i = 0; i < s->params.update; ++i) {
-            if (na > 0) M16_CUDA_TRY(launch_pdl(bt1_flow_kernel<kAlphaArray>, dim3(na), block, st, true, dwork, dvols,
-                                                dgroups, (const unsigned *)dmask));
-            if (ne > 0) M16_CUDA_TRY(launch_pdl(bt1_flow_kernel<kAlphaFromGrad2>, dim3(ne), block, st, true,
-                                                dwork + na, dvols, dgroups, (const unsigned *)dmask));
-            if (i == 0) {
-                M16_CUDA_TRY(launch_pdl(bt1_label_kernel<true>, dim3(s->n_items), block, st, true, dwork, dvols,
-                                        dgroups, (const unsigned *)dmask, dpart));
-                M16_CUDA_TRY(launch_pdl(bt_check_kernel, dim3(s->n_list), dim3(256), st, true, dvols, dgroups,
-                                        dinsts, dctrl, dmask, (const float4 *)dpart, s->params.error_bound,
-                                        s->params.update, dlist));
-            } else {
-                M16_CUDA_TRY(launch_pdl(bt1_label_kernel<false>, dim3(s->n_items), block, st, true, dwork, dvols,
-                                        dgroups, (const unsigned *)dmask, dpart));
-            }
+        int launches = 0;
+        std::copy(s->seg[0], s->seg[0] + kKinds + 1, B.seg);
+        if (s->n_full > 0) {
+            const int sweeps = enqueue_iterations(B, s->params.update, true, st, launches);
+            if (sweeps < 0) return M16_ERR_CUDA;
+            M16_CUDA_TRY(launch_check(s, B, s->n_full, (const int *)(s->ws + s->T.list), 0, sweeps & 1));
         }
+        std::copy(s->seg[1], s->seg[1] + kKinds + 1, B.seg);
+        if (s->n_list > s->n_full && enqueue_iterations(B, s->params.update - 1, false, st, launches) < 0)
+            return M16_ERR_CUDA;
         M16_CUDA_TRY(cudaGetLastError());
         M16_CUDA_TRY(cudaEventRecord(s->t_end[b], st));
         M16_CUDA_TRY(cudaEventRecord(s->step_end[b], st));
-        M16_CUDA_TRY(cudaMemcpyAsync(s->ctrl_h[b], dctrl, sizeof(InstCtrl) * s->max_slots, cudaMemcpyDeviceToHost,
+        M16_CUDA_TRY(cudaMemcpyAsync(s->ctrl_h[b], B.ctrl, sizeof(InstCtrl) * s->max_slots, cudaMemcpyDeviceToHost,
                                      st));
+        M16_CUDA_TRY(cudaMemcpyAsync(s->err_h + b, s->ws + s->T.err, sizeof(int), cudaMemcpyDeviceToHost, st));
         M16_CUDA_TRY(cudaEventRecord(s->ctrl_ev[b], st));
-        s->step_list[b] = s->list_cur;
+        s->step_list[b].clear();
         for (int k : s->list_cur) {
             Slot &sl = s->slots[k];
-            sl.iters_planned += s->params.update;
+            const bool full = full_step(s, sl);
+            sl.iters_planned += full ? s->params.update : s->params.update - 1;
+            sl.done_planning = !full;
             sl.last_listed = c;
-            if (sl.iters_planned >= s->params.num_iter) s->dirty = true;   // out of the next list
+            if (!full || !full_step(s, sl)) s->dirty = true;   // out of the next list, or in its other part
+            s->step_list[b].push_back({k, sl.iters_planned});
         }
         s->steps = c + 1;
     }
