@@ -3,16 +3,16 @@
 // kernels (src/clcode/gvf.cl:44-253) and of the loop in GvfGpu._execute
 // (src/processing/gradient_vector_flow.py:179-232).
 //
-// One fused sweep per iteration: g_out = g - dt * (r * (g - v) - mu * lap(g))
-// with the 7-point mirror-boundary Laplacian, reading g from one planar
-// buffer and writing the other (ping-pong), r = |v|^2 recomputed from v (or
-// read when the caller gives a response).  On check iterations the sweep
-// also sums |delta| per block for the convergence criterion.
+// One iteration: g_out = g - dt * (r * (g - v) - mu * lap(g)) with the 7-point
+// mirror-boundary Laplacian, r = |v|^2 recomputed from v (or read when the
+// caller gives a response).  gvf_tile.cuh runs several iterations per pass over
+// memory, alternating between two copies of g; volumes beyond 32-bit indexes
+// take the sweep of one iteration below.  On check iterations |delta| is summed
+// per block for the convergence criterion.
 //
 // Workspace: v0, v1, v2 (planar copies of the interleaved field), r (only
 // with a caller response), g_a[3], g_b[3], block partials, control word,
-// magnitude log.  Per voxel-iteration the sweep moves g 12 + v 12 (+ r 4)
-// read and g 12 written.
+// magnitude log.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -27,7 +27,9 @@ struct GvfCtrl {
     int stopped;
     int iterations;
     int n_checks;
-    int pad;
+    int buf;          // tile sweeps: the buffer that holds the field
+    int error;        // a copy of theirs did not arrive in time
+    int pad[3];
 };
 
 struct GvfArgs {
@@ -59,6 +61,8 @@ __global__ void gvf_init_kernel(const float *__restrict__ v3, const float *__res
         ctrl->stopped = 0;
         ctrl->iterations = 0;
         ctrl->n_checks = 0;
+        ctrl->buf = 0;
+        ctrl->error = 0;
     }
 }
 
@@ -277,12 +281,284 @@ inline GvfLayout gvf_layout(int d0, int d1, int d2, int has_response, int mags_c
 }  // namespace
 }  // namespace m16
 
+#include "gvf_tile.cuh"
+
+namespace m16 {
+namespace {
+
+// planar padded copies of the field, g = 0 in the first buffer
+__global__ void gvf_tile_init_kernel(const float *__restrict__ v3, const float *__restrict__ resp, int d2,
+                                     int64_t rows, float *__restrict__ v, float *__restrict__ r,
+                                     float *__restrict__ g, GvfCtrl *ctrl)
+{
+    const int pitch = tile_pitch(d2);
+    const int64_t np = rows * pitch;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < np; o += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = o / pitch;
+        const int x = (int)(o - row * pitch);
+        const bool in = x < d2;
+        const int64_t i = row * d2 + (in ? x : 0);
+        for (int c = 0; c < 3; ++c) {
+            v[c * np + o] = in ? v3[3 * i + c] : 0.f;
+            g[c * np + o] = 0.f;
+        }
+        if (resp) r[o] = in ? resp[i] : 0.f;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ctrl = GvfCtrl{0, 0, 0, 0, 0, {0, 0, 0}};
+}
+
+// mean |delta| of those of the iterations first .. first + count - 1 that are
+// checks, and the tolerance test (gradient_vector_flow.py:459-478)
+__global__ void gvf_tile_check_kernel(const float *__restrict__ part, int nparts, double inv_n, double tol, int first,
+                                      int count, int update, int cap, GvfCtrl *ctrl, double *mags)
+{
+    __shared__ double s[256];
+    pdl_wait();
+    pdl_launch_next();
+    if (__ldcg(&ctrl->stopped)) return;
+    for (int k = 0; k < count; ++k) {
+        const int it = first + k;
+        if (it % update) continue;
+        double acc = 0.0;
+        for (int j = threadIdx.x; j < nparts; j += blockDim.x) acc += (double)part[k * nparts + j];
+        s[threadIdx.x] = acc;
+        __syncthreads();
+        for (int w = blockDim.x >> 1; w > 0; w >>= 1) {
+            if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+            __syncthreads();
+        }
+        const double mag = s[0] * inv_n;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int idx = it / update;
+            if (idx < cap) mags[idx] = mag;
+            ctrl->n_checks = idx + 1;
+            if (mag < tol) {
+                ctrl->stopped = 1;
+                ctrl->iterations = it + 1;
+            }
+        }
+        if (mag < tol) return;   // uniform
+    }
+}
+
+// interleave (and optionally normalise, gvf.cl:215-232) the current field
+__global__ void gvf_tile_output_kernel(const float *__restrict__ g, int d2, int64_t rows, int normalize, int buf,
+                                       GvfCtrl *ctrl, float *__restrict__ g3)
+{
+    const int pitch = tile_pitch(d2);
+    const int64_t np = rows * pitch, n = rows * d2;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t o = i / d2 * pitch + i % d2;
+        float a = g[o], b = g[np + o], c = g[2 * np + o];
+        if (normalize) {
+            float nrm = sqrtf(a * a + b * b + c * c);
+            if (nrm != 0.f) {
+                nrm = 1.f / nrm;
+                a *= nrm; b *= nrm; c *= nrm;
+            }
+        }
+        g3[3 * i] = a;
+        g3[3 * i + 1] = b;
+        g3[3 * i + 2] = c;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->buf = buf;
+}
+
+struct GvfTileLayout {
+    size_t v, r, g[2], partials, ctrl, mags, total;
+    int cap;
+};
+
+// blocks of a launch of k iterations
+struct GvfTileGrid {
+    int nx, ny, zc, blocks;
+};
+
+inline GvfTileGrid gvf_tile_grid(int d0, int d1, int d2, int k)
+{
+    const int ow = kTileLanes - 2 * gvf_halo(k), oh = kGvfRows - 2 * (k - 1);
+    GvfTileGrid G;
+    G.nx = d2 <= kTileLanes ? 1 : (int)div_up(d2 - kTileLanes, ow) + 1;
+    G.ny = d1 <= kGvfRows ? 1 : (int)div_up(d1 - kGvfRows, oh) + 1;
+    const int64_t tiles = (int64_t)G.nx * G.ny, slots = (int64_t)kGvfBlocks * kSMs;
+    // least waves x marched planes (2 k + 1 of them beyond the block's own)
+    int64_t cost = INT64_MAX;
+    G.zc = 1;
+    for (int nz = 1; nz <= std::min(d0, 4096); ++nz) {
+        const int zc = (int)div_up(d0, nz);
+        const int64_t c = div_up(tiles * div_up(d0, zc), slots) * (zc + 2 * k + 1);
+        if (c < cost) {
+            cost = c;
+            G.zc = zc;
+        }
+        if (zc == 1) break;
+    }
+    G.blocks = (int)(tiles * div_up(d0, G.zc));
+    return G;
+}
+
+inline bool gvf_tile_ok(int d0, int d1, int d2) { return d2 >= 2 && tile_shape_ok(d0, d1, d2); }
+
+inline GvfTileLayout gvf_tile_layout(int d0, int d1, int d2, int has_response, int mags_cap)
+{
+    GvfTileLayout L;
+    const size_t np = (size_t)tile_voxels(d0, d1, d2);
+    L.cap = std::max(mags_cap, 1);
+    size_t off = 0, parts = 0;
+    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
+    L.v = take(3 * np * 4);
+    L.r = has_response ? take(np * 4) : 0;
+    for (int b = 0; b < 2; ++b) L.g[b] = take(3 * np * 4);
+    for (int k = 1; k <= kGvfK; ++k) parts = std::max(parts, (size_t)k * gvf_tile_grid(d0, d1, d2, k).blocks);
+    L.partials = take(parts * 4);
+    L.ctrl = take(sizeof(GvfCtrl));
+    L.mags = take((size_t)L.cap * 8);
+    L.total = off;
+    return L;
+}
+
+// tensor map of a padded planar field of three components: x, y, z, component
+inline bool gvf_map(CUtensorMap *m, const void *base, int d0, int d1, int pitch, int width, int rows)
+{
+    const cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)d1, (cuuint64_t)d0, 3};
+    const cuuint64_t row = (cuuint64_t)pitch * 4, strides[3] = {row, row * d1, row * d1 * d0};
+    const cuuint32_t box[4] = {(cuuint32_t)width, (cuuint32_t)rows, 1, 3};
+    return tile_map_encode(m, base, 4, dims, strides, box);
+}
+
+typedef void (*GvfTileKernel)(const GvfTileArgs);
+
+template <int K, bool RESP>
+GvfTileKernel gvf_kernel_of(bool check, bool flat)
+{
+    if (check) return flat ? gvf_tile_kernel<K, RESP, true, true> : gvf_tile_kernel<K, RESP, true, false>;
+    return flat ? gvf_tile_kernel<K, RESP, false, true> : gvf_tile_kernel<K, RESP, false, false>;
+}
+
+template <int K>
+GvfTileKernel gvf_kernel(int k, bool resp, bool check, bool flat, size_t *smem)
+{
+    if (k < K) return gvf_kernel<(K > 1 ? K - 1 : 1)>(k, resp, check, flat, smem);
+    *smem = resp ? sizeof(GvfMem<K, true>) : sizeof(GvfMem<K, false>);
+    return resp ? gvf_kernel_of<K, true>(check, flat) : gvf_kernel_of<K, false>(check, flat);
+}
+
+int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2, const double *voxel_size, double mu,
+                  double dt, int first_iter, int n_iters, int update, double tol, int normalize, float *g3,
+                  int32_t *iterations, int32_t *stopped, double *mags, int32_t mags_cap, int32_t *n_mags,
+                  const GvfTileLayout &L, char *ws, cudaStream_t st)
+{
+    const int64_t n = (int64_t)d0 * d1 * d2, rows = (int64_t)d0 * d1;
+    GvfCtrl *ctrl = (GvfCtrl *)(ws + L.ctrl);
+    double *mlog = (double *)(ws + L.mags);
+    float *g[2] = {(float *)(ws + L.g[0]), (float *)(ws + L.g[1])};
+    const int blocks1d = (int)std::min<int64_t>(4 * kSMs, div_up(n, 256));
+    GvfCtrl h = {};
+    if (first_iter == 0) {
+        gvf_tile_init_kernel<<<blocks1d, 256, 0, st>>>(v3, response, d2, rows, (float *)(ws + L.v),
+                                                       (float *)(ws + L.r), g[0], ctrl);
+        M16_CUDA_TRY(cudaGetLastError());
+    } else {
+        M16_CUDA_TRY(cudaMemcpyAsync(&h, ctrl, sizeof(h), cudaMemcpyDeviceToHost, st));
+        M16_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    const int buf0 = h.buf & 1;
+    const bool was_stopped = h.stopped != 0;
+    GvfTileArgs a = {};
+    a.d0 = d0; a.d1 = d1; a.d2 = d2; a.pitch = tile_pitch(d2);
+    a.rss0 = (float)(1.0 / (voxel_size[0] * voxel_size[0]));
+    a.rss1 = (float)(1.0 / (voxel_size[1] * voxel_size[1]));
+    a.rss2 = (float)(1.0 / (voxel_size[2] * voxel_size[2]));
+    a.nmu = -(float)mu;
+    a.ndt = -(float)dt;
+    a.comp = tile_voxels(d0, d1, d2);
+    a.partials = (float *)(ws + L.partials);
+    a.err = &ctrl->error;
+    CUtensorMap mg[2];
+    bool ok = gvf_map(&a.mv, ws + L.v, d0, d1, a.pitch, kGvfVW, kGvfRows);
+    for (int b = 0; b < 2; ++b) ok = ok && gvf_map(&mg[b], g[b], d0, d1, a.pitch, kGvfGW, kGvfRows + 2);
+    if (response) {
+        const cuuint64_t dims[3] = {(cuuint64_t)a.pitch, (cuuint64_t)d1, (cuuint64_t)d0};
+        const cuuint64_t row = (cuuint64_t)a.pitch * 4, strides[2] = {row, row * d1};
+        const cuuint32_t box[3] = {kGvfVW, kGvfRows, 1};
+        ok = ok && tile_map_encode(&a.mr, ws + L.r, 3, dims, strides, box);
+    }
+    if (!ok) return M16_ERR_CUDA;
+    GvfTileKernel kernels[kGvfK + 1][2];
+    size_t smem[kGvfK + 1];
+    GvfTileGrid grids[kGvfK + 1];
+    for (int k = 1; k <= kGvfK; ++k) {
+        grids[k] = gvf_tile_grid(d0, d1, d2, k);
+        for (int c = 0; c < 2; ++c) {
+            kernels[k][c] = gvf_kernel<kGvfK>(k, response != nullptr, c != 0, d1 < kGvfRows, &smem[k]);
+            M16_CUDA_TRY(
+                cudaFuncSetAttribute(kernels[k][c], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[k]));
+        }
+    }
+    // iterations it .. it + k - 1 from buffer b to the other
+    auto sweep = [&](int it, int k, int b, bool always) -> cudaError_t {
+        const GvfTileGrid &G = grids[k];
+        GvfTileArgs s = a;
+        s.mg = mg[b];
+        s.gi = g[b];
+        s.go = g[1 - b];
+        s.nx = G.nx; s.ny = G.ny; s.zc = G.zc;
+        s.ctrl = always ? nullptr : ctrl;
+        s.checks = 0;
+        if (!always)
+            for (int j = 0; j < k; ++j) s.checks |= (it + j) % update == 0 ? 1 << j : 0;
+        cudaError_t e = launch_pdl_smem(kernels[k][s.checks != 0], dim3(G.blocks), dim3(kTileLanes, kGvfNW), smem[k], st, true, s);
+        if (e == cudaSuccess && s.checks)
+            e = launch_pdl(gvf_tile_check_kernel, dim3(1), dim3(256), st, true, (const float *)a.partials, G.blocks,
+                           1.0 / (double)n, tol, it, k, update, L.cap, ctrl, mlog);
+        return e;
+    };
+    // programmatic dependent launch: each sweep waits on the device for the
+    // previous one (which reads the buffer it writes) before any access
+    int sweeps = 0;
+    for (int done = 0; done < n_iters; ++sweeps) {
+        const int k = std::min(kGvfK, n_iters - done);
+        M16_CUDA_TRY(sweep(first_iter + done, k, (buf0 + sweeps) & 1, false));
+        done += k;
+    }
+    M16_CUDA_TRY(cudaGetLastError());
+    M16_CUDA_TRY(cudaMemcpyAsync(&h, ctrl, sizeof(h), cudaMemcpyDeviceToHost, st));
+    M16_CUDA_TRY(cudaStreamSynchronize(st));
+    if (h.error) return M16_ERR_TIMEOUT;
+    const int done = h.stopped ? h.iterations : first_iter + n_iters;   // total iterations so far
+    int buf = buf0;
+    if (!was_stopped) {
+        const int ran = done - first_iter;
+        buf = (buf0 + (int)div_up(ran, kGvfK)) & 1;
+        // stopped inside a sweep: its iterations up to there again, from the
+        // buffer it read
+        if (h.stopped && ran % kGvfK && ran < n_iters)
+            M16_CUDA_TRY(sweep(done - ran % kGvfK, ran % kGvfK, 1 - buf, true));
+    }
+    gvf_tile_output_kernel<<<blocks1d, 256, 0, st>>>(g[buf], d2, rows, normalize, buf, ctrl, g3);
+    M16_CUDA_TRY(cudaGetLastError());
+    if (iterations) *iterations = done;
+    if (stopped) *stopped = h.stopped;
+    if (n_mags) *n_mags = h.n_checks;
+    if (mags && mags_cap > 0) {
+        const int cnt = std::min(std::min(h.n_checks, mags_cap), L.cap);
+        if (cnt > 0) M16_CUDA_TRY(cudaMemcpyAsync(mags, mlog, (size_t)cnt * 8, cudaMemcpyDeviceToHost, st));
+    }
+    M16_CUDA_TRY(cudaStreamSynchronize(st));
+    return M16_OK;
+}
+
+}  // namespace
+}  // namespace m16
+
 using namespace m16;
 
 extern "C" size_t m16_gvf_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, int32_t has_response,
                                           int32_t mags_cap)
 {
     if (d0 < 1 || d1 < 1 || d2 < 1) return 0;
+    if (gvf_tile_ok(d0, d1, d2)) return gvf_tile_layout(d0, d1, d2, has_response, mags_cap).total;
     return gvf_layout(d0, d1, d2, has_response, mags_cap).total;
 }
 
@@ -298,6 +574,13 @@ extern "C" int m16_gvf_run(const float *v3, const float *response, int32_t d0, i
     if (update < 1 || first_iter < 0 || n_iters < 0 || !(dt > 0.0) || !(mu >= 0.0)) return M16_ERR_BAD_ARG;
     for (int k = 0; k < 3; ++k)
         if (!(voxel_size[k] > 0.0)) return M16_ERR_BAD_ARG;
+    if (gvf_tile_ok(d0, d1, d2)) {
+        const GvfTileLayout T = gvf_tile_layout(d0, d1, d2, response != nullptr, mags_cap);
+        if (!workspace || workspace_bytes < T.total || ((uintptr_t)workspace & 255)) return M16_ERR_WORKSPACE;
+        return gvf_run_tiles(v3, response, d0, d1, d2, voxel_size, mu, dt, first_iter, n_iters, update, tol, normalize,
+                             g3, iterations, stopped, mags, mags_cap, n_mags, T, (char *)workspace,
+                             (cudaStream_t)stream);
+    }
     const GvfLayout L = gvf_layout(d0, d1, d2, response != nullptr, mags_cap);
     if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255)) return M16_ERR_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
