@@ -558,7 +558,9 @@ size_t m16_ridge_forest_joins_workspace_bytes(int64_t num_points);
  * is found exactly (integer squared distances, ties to the lowest indices);
  * the search compares every tree's points with those of the trees ranked
  * below it by size, and returns M16_ERR_TOO_LARGE, writing nothing, when that
- * takes more than max_pair_evaluations distance evaluations.  join_a, join_b
+ * takes more than max_pair_evaluations distance evaluations, or when there
+ * are more than 2^24 pairs of trees and more than 4 num_points (tree, point)
+ * combinations.  join_a, join_b
  * (host int32, capacity num_points - 1), *num_joins (host): the joining
  * edges, the lower index first.  Synchronizes `stream`.
  */

@@ -390,8 +390,12 @@ extern "C" int m16_ridge_signs(int64_t num_points, const int32_t *edges_a, const
 namespace m16 {
 namespace {
 
-constexpr int kFjChunk = 2048;          // target points per block, staged in shared memory
+constexpr int kFjChunk = 256;           // target points per block, staged in shared memory (a block a chunk: with
+                                        // 2048 a tree of a few thousand points kept one or two SMs busy)
 constexpr int kFjScanItems = 1024;      // points per block of the component numbering
+constexpr int64_t kFjMinKeys = 1 << 17;    // least keys of a group (1 MiB): a cleaned ridge of about 30 trees and 770
+                                           // points (22,000 keys) needs one group
+constexpr int64_t kFjMaxPairs = 1 << 24;   // pairs of trees in the host's list (20 bytes each)
 constexpr int64_t kFjMaxCoord = 32767;  // |dz|^2 + |dy|^2 + |dx|^2 < 2^32
 
 // roots per block of kFjScanItems points (a root is its component's lowest
@@ -478,12 +482,12 @@ struct FjChunk {
 };
 
 // every query point q of a rank above the chunk's against the chunk's points:
-// key[chunk rank][q - qbase] = min over targets p of (d^2 << 32 | p)
+// key[chunk rank - t0][q - qbase] = min over targets p of (d^2 << 32 | p)
 __global__ void __launch_bounds__(256) fj_nearest_kernel(const int32_t *__restrict__ pts,
                                                          const int32_t *__restrict__ perm,
                                                          const unsigned *__restrict__ start,
-                                                         const FjChunk *__restrict__ chunks, int64_t R, int64_t qbase,
-                                                         unsigned long long *__restrict__ key)
+                                                         const FjChunk *__restrict__ chunks, int32_t t0, int64_t R,
+                                                         int64_t qbase, unsigned long long *__restrict__ key)
 {
     __shared__ int4 tp[kFjChunk];
     const FjChunk ch = chunks[blockIdx.x];
@@ -494,7 +498,7 @@ __global__ void __launch_bounds__(256) fj_nearest_kernel(const int32_t *__restri
     }
     __syncthreads();
     const int64_t q0 = start[ch.rank + 1];
-    unsigned long long *krow = key + (int64_t)ch.rank * (R - qbase);
+    unsigned long long *krow = key + (int64_t)(ch.rank - t0) * (R - qbase);
     for (int64_t qi = q0 + threadIdx.x; qi < R; qi += blockDim.x) {
         const int32_t q = perm[qi];
         const int a = pts[3 * q], b = pts[3 * q + 1], c = pts[3 * q + 2];
@@ -510,6 +514,49 @@ __global__ void __launch_bounds__(256) fj_nearest_kernel(const int32_t *__restri
     }
 }
 
+// the least (d^2, lo, hi) between rank t0 + row and rank s > t0 + row, one
+// warp a pair of ranks: pair[row * C + s] = (d^2, lo, hi).  Bound by latency
+// (a few keys a lane).  Measured on a cleaned ridge of 770 points in about 30
+// trees, local phase and joins: 3.3 ms with k-d trees on the host (its 22,000
+// keys exceeded the 4 R that the walk over every key on the host was allowed),
+// 0.85 ms with this kernel and groups of ranks.
+__global__ void __launch_bounds__(256) fj_pair_kernel(const int32_t *__restrict__ perm,
+                                                      const unsigned *__restrict__ start, int32_t t0, int32_t rows,
+                                                      int32_t C, int64_t R, int64_t qbase,
+                                                      const unsigned long long *__restrict__ key,
+                                                      uint4 *__restrict__ pair)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5), n = (int64_t)rows * C;
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n; w += stride) {
+        const int32_t row = (int32_t)(w / C), s = (int32_t)(w - (int64_t)row * C);
+        if (s <= t0 + row) continue;
+        const unsigned long long *krow = key + (int64_t)row * (R - qbase);
+        unsigned long long best = ~0ull;   // d^2 << 32 | lo
+        unsigned hi = ~0u;
+        for (int64_t qi = (int64_t)start[s] + lane; qi < (int64_t)start[s + 1]; qi += 32) {
+            const unsigned long long k = krow[qi - qbase];
+            const unsigned q = (unsigned)perm[qi], p = (unsigned)k;
+            const unsigned long long m = (k & ~0xffffffffull) | min(q, p);
+            const unsigned h = max(q, p);
+            if (m < best || (m == best && h < hi)) {
+                best = m;
+                hi = h;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long m = __shfl_xor_sync(0xffffffffu, best, o);
+            const unsigned h = __shfl_xor_sync(0xffffffffu, hi, o);
+            if (m < best || (m == best && h < hi)) {
+                best = m;
+                hi = h;
+            }
+        }
+        if (lane == 0) pair[w] = make_uint4((unsigned)(best >> 32), (unsigned)best, hi, 0u);
+    }
+}
+
 __global__ void fj_fill_kernel(unsigned long long *p, int64_t n)
 {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
@@ -517,7 +564,7 @@ __global__ void fj_fill_kernel(unsigned long long *p, int64_t n)
 }
 
 struct FjLayout {
-    size_t parent, root, par, cid, comp, size, rank, start, fill, perm, bcount, chunks, key, ctrl, total;
+    size_t parent, root, par, cid, comp, size, rank, start, fill, perm, bcount, chunks, key, pair, ctrl, total;
     int64_t max_keys, max_chunks;
 };
 
@@ -531,7 +578,7 @@ FjLayout fj_layout(int64_t R)
         return o;
     };
     const int64_t nb = div_up(R, kFjScanItems);
-    L.max_keys = 4 * R;
+    L.max_keys = std::max<int64_t>(4 * R, kFjMinKeys);
     L.max_chunks = R / kFjChunk + R + 1;
     L.parent = take(4 * (size_t)R);
     L.root = take(4 * (size_t)R);
@@ -546,6 +593,7 @@ FjLayout fj_layout(int64_t R)
     L.bcount = take(4 * (size_t)nb);
     L.chunks = take(sizeof(FjChunk) * (size_t)L.max_chunks);
     L.key = take(8 * (size_t)L.max_keys);
+    L.pair = take(sizeof(uint4) * (size_t)L.max_keys);
     L.ctrl = take(32);
     L.total = off;
     return L;
@@ -587,6 +635,7 @@ extern "C" int m16_ridge_forest_joins(const int32_t *pts3, int64_t num_points, c
     unsigned *bcount = (unsigned *)(ws + Ly.bcount);
     FjChunk *chunks = (FjChunk *)(ws + Ly.chunks);
     unsigned long long *key = (unsigned long long *)(ws + Ly.key);
+    uint4 *pair = (uint4 *)(ws + Ly.pair);
     unsigned long long *ctrl = (unsigned long long *)(ws + Ly.ctrl);   // [0] walks at the limit, [1] bad edges, [2] bad coordinates
     const int gr = rs_grid(R), ge = rs_grid(std::max<int64_t>(num_edges, 1));
     const int64_t nb = div_up(R, kFjScanItems);
@@ -629,53 +678,56 @@ extern "C" int m16_ridge_forest_joins(const int32_t *pts3, int64_t num_points, c
         rank_h[order[t]] = (int32_t)t;
         hstart[t + 1] = hstart[t] + hsize[order[t]];
     }
-    // the work and memory of the search: every rank against the ranks after it
+    // the work of the search: every rank against the ranks after it
     const int64_t qbase = hstart[1];
     double work = 0.0;
     std::vector<FjChunk> hch;
+    std::vector<size_t> first_chunk(C, 0);   // of every rank but the last; [C - 1] the end
     for (unsigned t = 0; t + 1 < C; ++t) {
         work += (double)hsize[order[t]] * (double)(R - hstart[t + 1]);
         for (int64_t b0 = hstart[t]; b0 < (int64_t)hstart[t + 1]; b0 += kFjChunk)
             hch.push_back(FjChunk{(int32_t)t, (int32_t)b0, (int32_t)std::min<int64_t>(b0 + kFjChunk, hstart[t + 1])});
+        first_chunk[t + 1] = hch.size();
     }
-    const int64_t nkeys = (int64_t)(C - 1) * (R - qbase);
-    if (work > (double)max_pair_evaluations || nkeys > Ly.max_keys || (int64_t)hch.size() > Ly.max_chunks ||
-        (int64_t)hch.size() > INT32_MAX)
+    // Ranks are taken in groups whose keys fit the workspace.  A search in one
+    // group of 4 R keys was always taken; one in several groups is taken while
+    // the host's list of pairs stays within kFjMaxPairs.
+    const int64_t nkeys = (int64_t)(C - 1) * (R - qbase), npairs = (int64_t)C * (C - 1) / 2;
+    if (work > (double)max_pair_evaluations || (nkeys > 4 * R && npairs > kFjMaxPairs) ||
+        (int64_t)hch.size() > Ly.max_chunks || (int64_t)hch.size() > INT32_MAX)
         return M16_ERR_TOO_LARGE;
     M16_CUDA_TRY(cudaMemcpyAsync(rank_of, rank_h.data(), 4 * (size_t)C, cudaMemcpyHostToDevice, st));
     M16_CUDA_TRY(cudaMemcpyAsync(start, hstart.data(), 4 * (size_t)(C + 1), cudaMemcpyHostToDevice, st));
     M16_CUDA_TRY(cudaMemcpyAsync(chunks, hch.data(), sizeof(FjChunk) * hch.size(), cudaMemcpyHostToDevice, st));
     M16_CUDA_TRY(cudaMemsetAsync(fill, 0, 4 * (size_t)C, st));
     fj_scatter_kernel<<<gr, kRsBlock, 0, st>>>(comp, R, rank_of, start, fill, perm);
-    fj_fill_kernel<<<rs_grid(nkeys), kRsBlock, 0, st>>>(key, nkeys);
-    fj_nearest_kernel<<<(unsigned)hch.size(), 256, 0, st>>>(pts3, perm, start, chunks, R, qbase, key);
     M16_CUDA_TRY(cudaGetLastError());
-    std::vector<unsigned long long> hkey(nkeys);
-    std::vector<int32_t> hperm(R - qbase);
-    M16_CUDA_TRY(cudaMemcpyAsync(hkey.data(), key, 8 * (size_t)nkeys, cudaMemcpyDeviceToHost, st));
-    M16_CUDA_TRY(cudaMemcpyAsync(hperm.data(), perm + qbase, 4 * (size_t)(R - qbase), cudaMemcpyDeviceToHost, st));
-    M16_CUDA_TRY(cudaStreamSynchronize(st));
     // least (d^2, lo, hi) of every pair of ranks (s > t)
     struct Cand {
-        uint64_t d2;
+        uint32_t d2;
         int32_t lo, hi, s, t;
     };
     std::vector<Cand> cand;
-    cand.reserve((size_t)C * (C - 1) / 2);
-    for (unsigned t = 0; t + 1 < C; ++t) {
-        const unsigned long long *krow = hkey.data() + (int64_t)t * (R - qbase);
-        for (unsigned s = t + 1; s < C; ++s) {
-            Cand best{~0ull, INT32_MAX, INT32_MAX, (int32_t)s, (int32_t)t};
-            for (int64_t qi = hstart[s]; qi < (int64_t)hstart[s + 1]; ++qi) {
-                const unsigned long long k = krow[qi - qbase];
-                const int32_t q = hperm[qi - qbase], p = (int32_t)(k & 0xffffffffu);
-                const uint64_t d2 = k >> 32;
-                const int32_t lo = std::min(q, p), hi = std::max(q, p);
-                if (d2 < best.d2 || (d2 == best.d2 && (lo < best.lo || (lo == best.lo && hi < best.hi))))
-                    best = Cand{d2, lo, hi, (int32_t)s, (int32_t)t};
+    cand.reserve((size_t)npairs);
+    // rows of a group: R - qbase keys and C pairs each (C - 1 <= R - qbase)
+    const int64_t group = std::max<int64_t>(1, std::min<int64_t>(C - 1, Ly.max_keys / std::max<int64_t>(R - qbase, C)));
+    std::vector<uint4> hpair((size_t)group * C);
+    for (int64_t t0 = 0; t0 + 1 < (int64_t)C; t0 += group) {
+        const int64_t rows = std::min<int64_t>(group, (int64_t)C - 1 - t0);
+        const size_t c0 = first_chunk[t0], c1 = first_chunk[t0 + rows];
+        fj_fill_kernel<<<rs_grid(rows * (R - qbase)), kRsBlock, 0, st>>>(key, rows * (R - qbase));
+        fj_nearest_kernel<<<(unsigned)(c1 - c0), 256, 0, st>>>(pts3, perm, start, chunks + c0, (int32_t)t0, R, qbase,
+                                                               key);
+        fj_pair_kernel<<<rs_grid(32 * rows * C), 256, 0, st>>>(perm, start, (int32_t)t0, (int32_t)rows, (int32_t)C, R,
+                                                               qbase, key, pair);
+        M16_CUDA_TRY(cudaGetLastError());
+        M16_CUDA_TRY(cudaMemcpyAsync(hpair.data(), pair, sizeof(uint4) * (size_t)(rows * C), cudaMemcpyDeviceToHost, st));
+        M16_CUDA_TRY(cudaStreamSynchronize(st));
+        for (int64_t row = 0; row < rows; ++row)
+            for (int64_t s = t0 + row + 1; s < (int64_t)C; ++s) {
+                const uint4 e = hpair[(size_t)(row * C + s)];
+                cand.push_back(Cand{e.x, (int32_t)e.y, (int32_t)e.z, (int32_t)s, (int32_t)(t0 + row)});
             }
-            cand.push_back(best);
-        }
     }
     // Kruskal over the components in (weight, lo, hi) order
     std::sort(cand.begin(), cand.end(), [](const Cand &a, const Cand &b) {
