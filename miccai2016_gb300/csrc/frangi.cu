@@ -19,6 +19,7 @@
 #include <float.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 
@@ -37,85 +38,136 @@ struct AxisTaps {
 // mirror-completed index with period 2 (n - 1) (convolve_naive.cl:25-63)
 __device__ __forceinline__ int mirror(int p, int n)
 {
+    const int q = abs(p);   // the boundary is symmetric about 0
+    if (q < n) return q;
     if (n == 1) return 0;
     const int period = 2 * (n - 1);
+    if (q <= period) return period - q;   // within one period: no division
     p %= period;
     if (p < 0) p += period;
     return p < n ? p : period - p;
 }
 
-inline int fr_zc(int d0, int d1, int d2)
-{
-    const int64_t cols = div_up(d2, kBX) * div_up(d1, kBY);
-    int64_t zc = (int64_t)d0 * cols / (8 * kSMs);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(8, zc));
-}
+// ---- passes 1 and 2 for any radius -------------------------------------------
+// The kernels for radii above kRunMaxR (below) and for more z planes than a
+// grid holds: kAnyRun outputs per thread along the convolved axis, the taps
+// taken kAnyTaps at a time, so that every loaded value serves kAnyRun outputs
+// and every tap too.  Each output accumulates its taps in the order j = 0..K-1
+// (tap K-1-j), as the specialised passes do.  Bound by latency and issue on a
+// small volume: at 45 x 61 x 83, radius 18 and 24, the y passes with one output
+// per thread took 44 us each, every tap waiting for its loads, and 30 us so.
+constexpr int kAnyRun = 4, kAnyTaps = 8;
+constexpr int kAnyBY = 4;   // rows of a block: small volumes have few threads, and smaller blocks spread them
 
-// ---- pass 1: z (axis 0), orders 0, 1, 2 ------------------------------------
-__global__ void __launch_bounds__(kBX * kBY) fr_conv_z_kernel(const float *__restrict__ img, float *__restrict__ z0,
-                                                              float *__restrict__ z1, float *__restrict__ z2, int d0,
-                                                              int d1, int d2, int zc, AxisTaps tp)
+// the kAnyRun + kAnyTaps - 1 inputs of one block of taps: col[m * stride],
+// m = first, first + 1, ..., mirrored into [0, n) unless inner (then only cut
+// at n - 1: what lies beyond the last tap is not used)
+__device__ __forceinline__ void any_load(const float *__restrict__ col, int64_t stride, int first, int n, bool inner,
+                                         float (&v)[kAnyRun + kAnyTaps - 1])
 {
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    if (x >= d2 || y >= d1) return;
-    const int za = blockIdx.z * zc, zb = min(za + zc, d0);
-    const int64_t s0 = (int64_t)d1 * d2;
-    const int64_t col = (int64_t)y * d2 + x;
-    const int r = tp.radius, K = 2 * r + 1;
-    for (int z = za; z < zb; ++z) {
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-        const bool inner = z - r >= 0 && z + r < d0;
-        for (int j = 0; j < K; ++j) {
-            const int m = inner ? z - r + j : mirror(z - r + j, d0);
-            const float v = __ldg(img + col + m * s0);
-            const int k = K - 1 - j;
-            a0 = fmaf(tp.t[0][k], v, a0);
-            a1 = fmaf(tp.t[1][k], v, a1);
-            a2 = fmaf(tp.t[2][k], v, a2);
-        }
-        const int64_t i = col + z * s0;
-        z0[i] = a0;
-        z1[i] = a1;
-        z2[i] = a2;
+#pragma unroll
+    for (int p = 0; p < kAnyRun + kAnyTaps - 1; ++p) {
+        const int m = inner ? min(first + p, n - 1) : mirror(first + p, n);
+        v[p] = __ldg(col + (int64_t)m * stride);
     }
 }
 
-// ---- pass 2: y (axis 1), the six products ----------------------------------
-__global__ void __launch_bounds__(kBX * kBY) fr_conv_y_kernel(const float *__restrict__ z0, const float *__restrict__ z1,
-                                                              const float *__restrict__ z2, float *__restrict__ six,
-                                                              int d0, int d1, int d2, int zc, AxisTaps tp)
+// acc[o] += t[jj] * v[o + jj] over the block's taps in order
+__device__ __forceinline__ void any_fma(const float (&t)[kAnyTaps], int nt, const float (&v)[kAnyRun + kAnyTaps - 1],
+                                        float (&acc)[kAnyRun])
+{
+#pragma unroll
+    for (int jj = 0; jj < kAnyTaps; ++jj)
+        if (jj < nt)
+#pragma unroll
+            for (int o = 0; o < kAnyRun; ++o) acc[o] = fmaf(t[jj], v[o + jj], acc[o]);
+}
+
+__device__ __forceinline__ void any_taps(const AxisTaps &tp, int order, int j0, int K, float (&t)[kAnyTaps])
+{
+#pragma unroll
+    for (int jj = 0; jj < kAnyTaps; ++jj) t[jj] = tp.t[order][max(K - 1 - j0 - jj, 0)];
+}
+
+// pass 1: z (axis 0), orders 0, 1, 2
+__global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_z_kernel(const float *__restrict__ img, float *__restrict__ z0,
+                                                                 float *__restrict__ z1, float *__restrict__ z2, int d0,
+                                                                 int d1, int d2, const __grid_constant__ AxisTaps tp)
 {
     const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    if (x >= d2 || y >= d1) return;
-    const int za = blockIdx.z * zc, zb = min(za + zc, d0);
+    if (x >= d2) return;
+    const int64_t s0 = (int64_t)d1 * d2;
+    const int r = tp.radius, K = 2 * r + 1;
+    const int za = blockIdx.z * kAnyRun;
+    for (int y = blockIdx.y * kAnyBY + threadIdx.y; y < d1; y += gridDim.y * kAnyBY) {
+        const int64_t col = (int64_t)y * d2 + x;
+        const bool inner = za - r >= 0 && za + kAnyRun - 1 + r < d0;
+        float acc[3][kAnyRun] = {};
+        for (int j0 = 0; j0 < K; j0 += kAnyTaps) {
+            float v[kAnyRun + kAnyTaps - 1], t[kAnyTaps];
+            any_load(img + col, s0, za - r + j0, d0, inner, v);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                any_taps(tp, k, j0, K, t);
+                any_fma(t, K - j0, v, acc[k]);
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < kAnyRun; ++o) {
+            if (za + o < d0) {
+                const int64_t i = col + (int64_t)(za + o) * s0;
+                z0[i] = acc[0][o];
+                z1[i] = acc[1][o];
+                z2[i] = acc[2][o];
+            }
+        }
+    }
+}
+
+// pass 2: y (axis 1), the six products; block row = kAnyRun rows of the volume
+__global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_y_kernel(const float *__restrict__ z0,
+                                                                 const float *__restrict__ z1,
+                                                                 const float *__restrict__ z2, float *__restrict__ six,
+                                                                 int d0, int d1, int d2,
+                                                                 const __grid_constant__ AxisTaps tp)
+{
+    const int x = blockIdx.x * kBX + threadIdx.x;
+    const int ya = (blockIdx.y * kAnyBY + threadIdx.y) * kAnyRun;
+    if (x >= d2 || ya >= d1) return;
     const int64_t s0 = (int64_t)d1 * d2, n = s0 * d0;
     const int r = tp.radius, K = 2 * r + 1;
-    const bool inner = y - r >= 0 && y + r < d1;
-    for (int z = za; z < zb; ++z) {
+    const bool inner = ya - r >= 0 && ya + kAnyRun - 1 + r < d1;
+    for (int z = blockIdx.z; z < d0; z += gridDim.z) {
         const int64_t plane = (int64_t)z * s0 + x;
-        float A = 0.f, B = 0.f, C = 0.f, D = 0.f, E = 0.f, F = 0.f;
-        for (int j = 0; j < K; ++j) {
-            const int m = inner ? y - r + j : mirror(y - r + j, d1);
-            const int64_t idx = plane + (int64_t)m * d2;
-            const float v0 = __ldg(z0 + idx), v1 = __ldg(z1 + idx), v2 = __ldg(z2 + idx);
-            const int k = K - 1 - j;
-            const float t0 = tp.t[0][k], t1 = tp.t[1][k], t2 = tp.t[2][k];
-            A = fmaf(t0, v2, A);
-            B = fmaf(t2, v0, B);
-            C = fmaf(t0, v0, C);
-            D = fmaf(t1, v1, D);
-            E = fmaf(t0, v1, E);
-            F = fmaf(t1, v0, F);
+        float A[kAnyRun] = {}, B[kAnyRun] = {}, C[kAnyRun] = {}, D[kAnyRun] = {}, E[kAnyRun] = {}, F[kAnyRun] = {};
+        for (int j0 = 0; j0 < K; j0 += kAnyTaps) {
+            const int first = ya - r + j0, nt = K - j0;
+            float v0[kAnyRun + kAnyTaps - 1], v1[kAnyRun + kAnyTaps - 1], v2[kAnyRun + kAnyTaps - 1], t[kAnyTaps];
+            any_load(z0 + plane, d2, first, d1, inner, v0);
+            any_load(z1 + plane, d2, first, d1, inner, v1);
+            any_load(z2 + plane, d2, first, d1, inner, v2);
+            any_taps(tp, 0, j0, K, t);
+            any_fma(t, nt, v2, A);   // A = y0 Z2
+            any_fma(t, nt, v0, C);   // C = y0 Z0
+            any_fma(t, nt, v1, E);   // E = y0 Z1
+            any_taps(tp, 1, j0, K, t);
+            any_fma(t, nt, v1, D);   // D = y1 Z1
+            any_fma(t, nt, v0, F);   // F = y1 Z0
+            any_taps(tp, 2, j0, K, t);
+            any_fma(t, nt, v0, B);   // B = y2 Z0
         }
-        const int64_t i = plane + (int64_t)y * d2;
-        six[i] = A;
-        six[n + i] = B;
-        six[2 * n + i] = C;
-        six[3 * n + i] = D;
-        six[4 * n + i] = E;
-        six[5 * n + i] = F;
+#pragma unroll
+        for (int o = 0; o < kAnyRun; ++o) {
+            if (ya + o < d1) {
+                const int64_t i = plane + (int64_t)(ya + o) * d2;
+                six[i] = A[o];
+                six[n + i] = B[o];
+                six[2 * n + i] = C[o];
+                six[3 * n + i] = D[o];
+                six[4 * n + i] = E[o];
+                six[5 * n + i] = F[o];
+            }
+        }
     }
 }
 
@@ -270,19 +322,34 @@ __device__ __forceinline__ float vesselness(const float e[6], float alpha, float
 
 struct FrArgs {
     int d0, d1, d2, zc;
-    float alpha, beta, c;   // c < 0: read the per-scale c from *c_dev
+    float alpha, beta, c;   // c < 0: from the scale's greatest Hessian norm
     int bright;
     const float *six;
     float *eig6;            // N x 6, or null when the update is fused
     float *val, *quat3;
-    float *partials;        // per-block max Hessian norm
-    const float *c_dev;     // the update kernel's scale's c
-    // c of the previous scale when its update rides along in this x pass
-    // (read from eig6 just before this scale's triple replaces it), else null
-    const float *c_prev;
+    int *norm;              // this scale's greatest Hessian norm (scale_c below)
+    // the norm of the previous scale when its update rides along in this x
+    // pass (read from eig6 just before this scale's triple replaces it), else null
+    const int *norm_prev;
     int first;              // the update done here is the first one: it writes
                             // val and quat without reading them
 };
+
+// A scale's greatest Hessian norm (calculateNorm + redMax) is kept as the bits
+// of the float, which order as integers do for norms >= 0; every block of the x
+// pass raises it with one atomicMax.  kNoNorm: no norm but NaN was seen.
+constexpr int kNoNorm = -1;
+
+// c = 0.5 * max norm of one scale (qfrangi_gpu.py:429-433)
+__host__ __device__ __forceinline__ float scale_c(int norm)
+{
+    union {
+        int i;
+        float f;
+    } u;
+    u.i = norm;
+    return 0.5f * (norm == kNoNorm ? NAN : u.f);
+}
 
 // one scale's update of the running maximum (updateVesselness,
 // frangi.cl:46-92).  The first update writes what the maximum over
@@ -316,7 +383,7 @@ __device__ __forceinline__ void x_output(const FrArgs &a, const float e[6], int6
         update_max(a, e, a.c, a.first != 0, i);
     } else {
         float2 *o = reinterpret_cast<float2 *>(a.eig6 + 6 * i);
-        if (a.c_prev) {
+        if (a.norm_prev) {
             const float2 p01 = o[0], p23 = o[1], p45 = o[2];
             const float ep[6] = {p01.x, p01.y, p23.x, p23.y, p45.x, p45.y};
             update_max(a, ep, c_prev, a.first != 0, i);
@@ -329,84 +396,32 @@ __device__ __forceinline__ void x_output(const FrArgs &a, const float e[6], int6
     }
 }
 
-template <bool FUSED_UPDATE>
-__device__ __forceinline__ void x_epilogue(const FrArgs &a, const float h[6], int64_t i, float c_prev, float &mx)
+// block maximum of the norms into the scale's (redMax, max.cl); fmaxf ignores
+// NaN as the reference's fmax does, and a block that saw nothing else adds nothing
+template <int WARPS>
+__device__ __forceinline__ void block_max_to_norm(float mx, float *red, int *norm)
 {
-    float e[6];
-    eig3(h, e);
-    x_output<FUSED_UPDATE>(a, e, i, c_prev, mx);
-}
-
-// block maximum of the norms into the block's partial (redMax, max.cl);
-// fmaxf ignores NaN as the reference's fmax does
-__device__ __forceinline__ void block_max_to_partial(float mx, float *red, float *partials)
-{
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    const int tid = threadIdx.x + kBX * threadIdx.y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
     if ((tid & 31) == 0) red[tid >> 5] = mx;
     __syncthreads();
     if (tid == 0) {
         float m = red[0];
-        for (int w = 1; w < (kBX * kBY) / 32; ++w) m = fmaxf(m, red[w]);
-        partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = m;
+        for (int w = 1; w < WARPS; ++w) m = fmaxf(m, red[w]);
+        if (m >= 0.f) atomicMax(norm, __float_as_int(m));
     }
-}
-
-// ---- pass 3: x (axis 2) fused with the eigensolve ----------------------------
-// One lane per voxel.  The Jacobi's data-dependent sweep count makes a warp
-// wait for its slowest voxel (21 of 32 lanes active on average).  Handing
-// each lane the next matrix of a per-warp pool as its own converges raised
-// that to 25 of 32 but added as many instructions as it saved (895 M -> 910
-// M warp instructions at 256^3, sigma 1, still issue-bound): no faster.
-// This is the kernel for any radius; radii up to kRunMaxR take the
-// specialised fr_conv_x_eig_run_kernel below.
-template <bool FUSED_UPDATE>
-__global__ void __launch_bounds__(kBX * kBY) fr_conv_x_eig_kernel(FrArgs a, AxisTaps tp)
-{
-    __shared__ float red[32];
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const float c_prev = (!FUSED_UPDATE && a.c_prev) ? *a.c_prev : 0.f;
-    float mx = -INFINITY;
-    if (x < a.d2 && y < a.d1) {
-        const int za = blockIdx.z * a.zc, zb = min(za + a.zc, a.d0);
-        const int64_t s0 = (int64_t)a.d1 * a.d2, n = s0 * a.d0;
-        const int r = tp.radius, K = 2 * r + 1;
-        const bool inner = x - r >= 0 && x + r < a.d2;
-        for (int z = za; z < zb; ++z) {
-            const int64_t row = (int64_t)z * s0 + (int64_t)y * a.d2;
-            float h[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int j = 0; j < K; ++j) {
-                const int m = inner ? x - r + j : mirror(x - r + j, a.d2);
-                const int64_t idx = row + m;
-                const int k = K - 1 - j;
-                const float t0 = tp.t[0][k], t1 = tp.t[1][k], t2 = tp.t[2][k];
-                h[0] = fmaf(t0, __ldg(a.six + idx), h[0]);
-                h[1] = fmaf(t0, __ldg(a.six + n + idx), h[1]);
-                h[2] = fmaf(t2, __ldg(a.six + 2 * n + idx), h[2]);
-                h[3] = fmaf(t0, __ldg(a.six + 3 * n + idx), h[3]);
-                h[4] = fmaf(t1, __ldg(a.six + 4 * n + idx), h[4]);
-                h[5] = fmaf(t1, __ldg(a.six + 5 * n + idx), h[5]);
-            }
-            x_epilogue<FUSED_UPDATE>(a, h, row + x, c_prev, mx);
-        }
-    }
-    if (!FUSED_UPDATE) block_max_to_partial(mx, red, a.partials);
 }
 
 // ---- radius-specialised passes ------------------------------------------------
 // For radii 1..kRunMaxR every pass is instantiated per radius: the tap loops
 // unroll and the taps become constant operands.  The z and y passes keep a
 // run of outputs per thread and read each input once for the whole run
-// (kRun + 2R loads instead of kRun * (2R + 1)); the x pass stages each row
-// of the six products, with its halo, in the warp's own shared memory and
-// convolves from there.  Every output still accumulates its taps in the
-// same order (j = 0..K-1, tap K-1-j) with the same fused multiply-adds, so
-// the results equal the kernels above bit for bit.
+// (kRun + 2R loads instead of kRun * (2R + 1)).  Every output accumulates its
+// taps in the same order (j = 0..K-1, tap K-1-j) with the same fused
+// multiply-adds at every radius, so the results do not depend on the kernel.
 constexpr int kRunMaxR = 16;
 constexpr int kRun = 8;   // outputs per thread along z (z pass) or y (y pass)
-static_assert(2 * kRunMaxR <= kBX, "the x pass stages each row in two 32-column steps");
 
 template <int R, bool INNER>
 __device__ __forceinline__ void z_run(const float *__restrict__ col, int64_t s0, int za, int d0, const AxisTaps &tp,
@@ -517,65 +532,137 @@ __global__ void __launch_bounds__(kBX * kBY) fr_conv_y_run_kernel(const float *_
     }
 }
 
-// x pass fused with the eigensolve; warp w of the block works on row
-// y = blockIdx.y * kBY + w and stages its 32 + 2R columns of the six
-// products in shared memory (only __syncwarp between staging and reads)
-template <bool FUSED_UPDATE, int R>
-__global__ void __launch_bounds__(kBX * kBY) fr_conv_x_eig_run_kernel(FrArgs a, AxisTaps tp)
+// ---- pass 3: x (axis 2) fused with the eigensolve ----------------------------
+// Warp w of a block works on kSeg = 128 columns of row y = blockIdx.y * warps
+// + w.  It stages the columns of the six products with their halo in its own
+// shared memory (only __syncwarp in between), convolves four neighbouring
+// columns per lane from 16-byte reads, puts the Hessians back through the same
+// memory, and solves them one column per lane, 32 neighbouring columns at a
+// time, so the results are written in order.
+//
+// Bound by issue in the eigensolve (4.9 Jacobi sweeps per warp at 256^3, about
+// 150 instructions each, and the squeeze).  With one column per lane the
+// convolution read 6 (2R + 1) floats of shared memory per column, one
+// wavefront per 32 columns each: 272 us of the radius-12 pass at 256^3 at one
+// wavefront a clock, which the eigensolve did not hide; four columns per lane
+// read 6 (2R + 4) / 4.  Measured at 256^3, radius 12 / 8 / 4: 752 / 699 / 577 us ->
+// 714 / 670 / 541 us; at 45 x 61 x 83, radius 18: 46 -> 24 us.
+//
+// The Jacobi's data-dependent sweep count makes a warp wait for its slowest
+// voxel (77 % of the lanes' sweeps are of use).  Handing each lane the next
+// matrix of a per-warp pool as its own converges raised that but added as many
+// instructions as it saved: no faster.
+//
+// R = 0 is the kernel for any radius, with its taps read from the parameters'
+// constant bank as it goes and its rows in dynamic shared memory.
+constexpr int kSeg = 128;    // columns of a warp
+constexpr int kXAnyBY = 4;   // warps of a block for any radius
+
+constexpr int fr_row_floats(int r) { return (kSeg + 2 * r + 3) / 4 * 4; }
+
+template <int R>
+__device__ __forceinline__ void x_conv4(const float *__restrict__ buf4, const float (&taps)[kMaxTaps], int radius,
+                                        float (&acc)[4])
 {
-    constexpr int K = 2 * R + 1, W = kBX + 2 * R;
-    __shared__ float red[32];
-    __shared__ float rows[kBY][6][W];
-    const int lane = threadIdx.x;
-    const int x0 = blockIdx.x * kBX, x = x0 + lane;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const float c_prev = (!FUSED_UPDATE && a.c_prev) ? *a.c_prev : 0.f;
-    float mx = -INFINITY;
-    if (y < a.d1) {   // uniform over the warp
-        float (*buf)[W] = rows[threadIdx.y];
-        const int za = blockIdx.z * a.zc, zb = min(za + a.zc, a.d0);
-        const int64_t s0 = (int64_t)a.d1 * a.d2, n = s0 * a.d0;
-        const bool inner = x0 - R >= 0 && x0 + kBX - 1 + R < a.d2;
-        for (int z = za; z < zb; ++z) {
-            const int64_t row = (int64_t)z * s0 + (int64_t)y * a.d2;
+    // output o of this lane: sum over j of taps[K - 1 - j] * buf4[o + j]
+    const int K = 2 * (R > 0 ? R : radius) + 1;
+    const float4 *p = reinterpret_cast<const float4 *>(buf4);
+    float w[8];
+    float4 q = p[0];
+    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+    w[4] = w[5] = w[6] = w[7] = 0.f;
 #pragma unroll
-            for (int i0 = 0; i0 < W; i0 += kBX) {
-                const int i = i0 + lane;
-                if (i < W) {
-                    const int m = inner ? x0 - R + i : mirror(x0 - R + i, a.d2);
-                    const float *src = a.six + row + m;
+    for (int o = 0; o < 4; ++o) acc[o] = 0.f;
+    if (R > 0) {
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) buf[c][i] = __ldg(src + c * n);
-                }
+        for (int j0 = 0; j0 < 2 * R + 1; j0 += 4) {
+            if (j0 + 1 < 2 * R + 1) {   // a last block of one tap needs no more columns, and the row ends there
+                q = p[j0 / 4 + 1];
+                w[4] = q.x; w[5] = q.y; w[6] = q.z; w[7] = q.w;
             }
-            __syncwarp();
-            float h[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const int k = K - 1 - j;
-                h[0] = fmaf(tp.t[0][k], buf[0][lane + j], h[0]);
-                h[1] = fmaf(tp.t[0][k], buf[1][lane + j], h[1]);
-                h[2] = fmaf(tp.t[2][k], buf[2][lane + j], h[2]);
-                h[3] = fmaf(tp.t[0][k], buf[3][lane + j], h[3]);
-                h[4] = fmaf(tp.t[1][k], buf[4][lane + j], h[4]);
-                h[5] = fmaf(tp.t[1][k], buf[5][lane + j], h[5]);
+            for (int jj = 0; jj < 4; ++jj)
+                if (j0 + jj < 2 * R + 1)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) acc[o] = fmaf(taps[2 * R - j0 - jj], w[o + jj], acc[o]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = w[k + 4];
+        }
+    } else {
+#pragma unroll 2
+        for (int j0 = 0; j0 < K; j0 += 4) {
+            if (j0 + 1 < K) {   // a last block of one tap needs no more columns, and the row ends there
+                q = p[j0 / 4 + 1];
+                w[4] = q.x; w[5] = q.y; w[6] = q.z; w[7] = q.w;
             }
-            __syncwarp();
-            // Every lane solves (a zero matrix past the volume's edge), and the
-            // warp meets again before the sort and squeeze: without that, lanes
-            // that finish their sweeps at different counts run the squeeze's
-            // atan2/acos in as many separate groups (about 3x its instructions).
-            if (x >= a.d2)
-                for (int c = 0; c < 6; ++c) h[c] = 0.f;
-            Jacobi J;
-            jacobi_sweeps(h, J);
-            __syncwarp();
-            float e[6];
-            jacobi_finish(J, e);
-            if (x < a.d2) x_output<FUSED_UPDATE>(a, e, row + x, c_prev, mx);
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj)
+                if (j0 + jj < K)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) acc[o] = fmaf(taps[K - 1 - j0 - jj], w[o + jj], acc[o]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = w[k + 4];
         }
     }
-    if (!FUSED_UPDATE) block_max_to_partial(mx, red, a.partials);
+}
+
+template <bool FUSED_UPDATE, int R>
+__global__ void __launch_bounds__(kBX * (R > 0 ? kBY : kXAnyBY)) fr_conv_x_eig_kernel(const __grid_constant__ FrArgs a,
+                                                                                      const __grid_constant__ AxisTaps tp)
+{
+    constexpr int kWarps = R > 0 ? kBY : kXAnyBY;
+    __shared__ float red[kWarps];
+    extern __shared__ __align__(16) float rows[];
+    const int lane = threadIdx.x, warp = threadIdx.y;
+    const int r = R > 0 ? R : tp.radius, W = fr_row_floats(r);
+    const int x0 = blockIdx.x * kSeg, cnt = min(kSeg, a.d2 - x0);
+    const float c_prev = (!FUSED_UPDATE && a.norm_prev) ? scale_c(*a.norm_prev) : 0.f;
+    float mx = -INFINITY;
+    float *buf = rows + (size_t)warp * 6 * W;
+    const int za = blockIdx.z * a.zc, zb = min(za + a.zc, a.d0);
+    for (int y = blockIdx.y * kWarps + warp; y < a.d1; y += gridDim.y * kWarps) {   // uniform over the warp
+        const int64_t s0 = (int64_t)a.d1 * a.d2, n = s0 * a.d0;
+        const int need = cnt + 2 * r;
+        const bool inner = x0 - r >= 0 && x0 + cnt + r <= a.d2;
+        for (int z = za; z < zb; ++z) {
+            const int64_t row = (int64_t)z * s0 + (int64_t)y * a.d2;
+            for (int i = lane; i < need; i += kBX) {
+                const int m = inner ? x0 - r + i : mirror(x0 - r + i, a.d2);
+                const float *src = a.six + row + m;
+#pragma unroll
+                for (int c = 0; c < 6; ++c) buf[c * W + i] = __ldg(src + c * n);
+            }
+            __syncwarp();
+            // columns past cnt convolve what the row holds there; nothing reads the result
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                constexpr int order[6] = {0, 0, 2, 0, 1, 1};
+                float acc[4];
+                x_conv4<R>(buf + c * W + 4 * lane, tp.t[order[c]], r, acc);
+                __syncwarp();
+                *reinterpret_cast<float4 *>(buf + c * W + 4 * lane) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int i = lane; i < kSeg && i - lane < cnt; i += kBX) {
+                // Every lane solves (a zero matrix past the volume's edge), and the
+                // warp meets again before the sort and squeeze: without that, lanes
+                // that finish their sweeps at different counts run the squeeze's
+                // atan2/acos in as many separate groups (about 3x its instructions).
+                float h[6];
+#pragma unroll
+                for (int c = 0; c < 6; ++c) h[c] = i < cnt ? buf[c * W + i] : 0.f;
+                Jacobi J;
+                jacobi_sweeps(h, J);
+                __syncwarp();
+                float e[6];
+                jacobi_finish(J, e);
+                if (i < cnt) x_output<FUSED_UPDATE>(a, e, row + x0 + i, c_prev, mx);
+            }
+            __syncwarp();
+        }
+    }
+    if (!FUSED_UPDATE) block_max_to_norm<kWarps>(mx, red, a.norm);
 }
 
 #define FR_RADIUS_CASES(CALL)                                                                                   \
@@ -585,40 +672,34 @@ __global__ void __launch_bounds__(kBX * kBY) fr_conv_x_eig_run_kernel(FrArgs a, 
     case 13: CALL(13); break; case 14: CALL(14); break; case 15: CALL(15); break; case 16: CALL(16); break;
 
 // the x pass for one scale: the specialised kernel for radii 1..kRunMaxR,
-// else the kernel for any radius (same grid)
+// else the kernel for any radius
 template <bool FUSED_UPDATE>
-void launch_x_eig(const FrArgs &a, const AxisTaps &tpx, dim3 grid, cudaStream_t st)
+cudaError_t launch_x_eig(const FrArgs &a, const AxisTaps &tpx, cudaStream_t st)
 {
-    const dim3 block(kBX, kBY, 1);
-#define FR_X_CALL(R) fr_conv_x_eig_run_kernel<FUSED_UPDATE, R><<<grid, block, 0, st>>>(a, tpx)
+    const bool any = tpx.radius < 1 || tpx.radius > kRunMaxR;
+    const int warps = any ? kXAnyBY : kBY;
+    const size_t smem = (size_t)warps * 6 * fr_row_floats(tpx.radius) * sizeof(float);
+    const dim3 block(kBX, warps, 1);
+    const dim3 grid((unsigned)div_up(a.d2, kSeg), (unsigned)std::min<int64_t>(65535, div_up(a.d1, warps)),
+                    (unsigned)div_up(a.d0, a.zc));
+#define FR_X_CALL(R) fr_conv_x_eig_kernel<FUSED_UPDATE, R><<<grid, block, smem, st>>>(a, tpx)
     switch (tpx.radius) {
         FR_RADIUS_CASES(FR_X_CALL)
-        default: fr_conv_x_eig_kernel<FUSED_UPDATE><<<grid, block, 0, st>>>(a, tpx); break;
+        default: FR_X_CALL(0); break;
     }
 #undef FR_X_CALL
+    return cudaGetLastError();
 }
-
-// c = 0.5 * max norm of one scale (qfrangi_gpu.py:429-433)
-__global__ void fr_c_kernel(const float *__restrict__ part, int nparts, float *c_out)
-{
-    __shared__ float s[256];
-    float m = -INFINITY;
-    for (int k = threadIdx.x; k < nparts; k += blockDim.x) m = fmaxf(m, part[k]);
-    s[threadIdx.x] = m;
-    __syncthreads();
-    for (int w = blockDim.x >> 1; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) s[threadIdx.x] = fmaxf(s[threadIdx.x], s[threadIdx.x + w]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *c_out = 0.5f * (s[0] == -INFINITY ? NAN : s[0]);
-}
+// the largest radius' rows fit the shared memory that a block has without asking
+static_assert(kXAnyBY * 6 * fr_row_floats((kMaxTaps - 1) / 2) * sizeof(float) + 64 <= 48 * 1024, "x pass rows");
+static_assert(kBY * 6 * fr_row_floats(kRunMaxR) * sizeof(float) + 64 <= 48 * 1024, "x pass rows");
 
 // updateVesselness (frangi.cl:46-92) of the last scale from its stored
 // eigendecompositions (the earlier scales' updates ride along in the next
 // scale's x pass)
 __global__ void fr_update_kernel(FrArgs a, int64_t n)
 {
-    const float c = *a.c_dev;
+    const float c = scale_c(*a.norm);
     const bool first = a.first != 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 *p = reinterpret_cast<const float2 *>(a.eig6 + 6 * i);
@@ -636,6 +717,13 @@ __global__ void fr_eigs_kernel(const float *__restrict__ in6, float *__restrict_
         eig3(h, e);
         for (int k = 0; k < 6; ++k) out6[6 * i + k] = e[k];
     }
+}
+
+inline int fr_zc(int d0, int d1, int d2)
+{
+    const int64_t cols = div_up(d2, kBX) * div_up(d1, kBY);
+    int64_t zc = (int64_t)d0 * cols / (8 * kSMs);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(8, zc));
 }
 
 // interleave the x-pass of the six products into an N x 6 Hessian (tests)
@@ -666,23 +754,19 @@ __global__ void fr_conv_x_hessian_kernel(const float *__restrict__ six, float *_
 }
 
 struct FrLayout {
-    size_t z, six, eig, part, cdev, total;
-    int nparts;
+    size_t z, six, eig, norm, total;
 };
 
 inline FrLayout fr_layout(int d0, int d1, int d2, int nscales)
 {
     FrLayout L;
     const int64_t n = (int64_t)d0 * d1 * d2;
-    const int zc = fr_zc(d0, d1, d2);
-    L.nparts = (int)(div_up(d2, kBX) * div_up(d1, kBY) * div_up(d0, zc));
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
     L.z = take(3 * n * 4);
     L.six = take(6 * n * 4);
     L.eig = take(6 * n * 4);
-    L.part = take((size_t)L.nparts * 4);
-    L.cdev = take((size_t)std::max(nscales, 1) * 4);
+    L.norm = take((size_t)std::max(nscales, 1) * 4);
     L.total = off;
     return L;
 }
@@ -704,25 +788,27 @@ int hessian_passes(const float *img, int d0, int d1, int d2, const float *taps, 
         !fill_taps(*tpx, taps + 6 * kMaxTaps, radius[2]))
         return M16_ERR_BAD_ARG;
     const int64_t n = (int64_t)d0 * d1 * d2;
-    const int zc = fr_zc(d0, d1, d2);
-    const dim3 block(kBX, kBY, 1);
-    const dim3 grid((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kBY), (unsigned)div_up(d0, zc));
+    const dim3 block(kBX, kBY, 1), block_any(kBX, kAnyBY, 1);
     float *z = (float *)(ws + L.z);
     float *six = (float *)(ws + L.six);
+    const dim3 any_z((unsigned)div_up(d2, kBX), (unsigned)std::min<int64_t>(65535, div_up(d1, kAnyBY)),
+                     (unsigned)div_up(d0, kAnyRun));
     const dim3 grid_z((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kBY), (unsigned)div_up(d0, kRun));
 #define FR_Z_CALL(R) fr_conv_z_run_kernel<R><<<grid_z, block, 0, st>>>(img, z, z + n, z + 2 * n, d0, d1, d2, tpz)
     switch (tpz.radius) {
         FR_RADIUS_CASES(FR_Z_CALL)
-        default: fr_conv_z_kernel<<<grid, block, 0, st>>>(img, z, z + n, z + 2 * n, d0, d1, d2, zc, tpz); break;
+        default: fr_conv_z_kernel<<<any_z, block_any, 0, st>>>(img, z, z + n, z + 2 * n, d0, d1, d2, tpz); break;
     }
 #undef FR_Z_CALL
+    const dim3 any_y((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kAnyBY * kAnyRun),
+                     (unsigned)std::min(65535, d0));
     // one z plane per block of the specialised y pass (grid z limit 65535)
     const dim3 grid_y((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kBY * kRun), (unsigned)d0);
     const int ry = d0 <= 65535 ? tpy.radius : 0;
 #define FR_Y_CALL(R) fr_conv_y_run_kernel<R><<<grid_y, block, 0, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, tpy)
     switch (ry) {
         FR_RADIUS_CASES(FR_Y_CALL)
-        default: fr_conv_y_kernel<<<grid, block, 0, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, zc, tpy); break;
+        default: fr_conv_y_kernel<<<any_y, block_any, 0, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, tpy); break;
     }
 #undef FR_Y_CALL
     M16_CUDA_TRY(cudaGetLastError());
@@ -753,37 +839,34 @@ extern "C" int m16_frangi(const float *img, int32_t d0, int32_t d1, int32_t d2, 
     const int64_t n = (int64_t)d0 * d1 * d2;
     const int blocks1d = (int)std::min<int64_t>(8 * kSMs, div_up(n, 256));
     FrArgs a;
-    a.d0 = d0; a.d1 = d1; a.d2 = d2; a.zc = fr_zc(d0, d1, d2);
+    a.d0 = d0; a.d1 = d1; a.d2 = d2; a.zc = (int)div_up(d0, 65535);
     a.alpha = alpha; a.beta = beta; a.c = c; a.bright = bright;
     a.six = (const float *)(ws + L.six);
     a.eig6 = (float *)(ws + L.eig);
     a.val = val; a.quat3 = quat3;
-    a.partials = (float *)(ws + L.part);
-    a.c_dev = nullptr;
-    a.c_prev = nullptr;
+    int *norm = (int *)(ws + L.norm);
+    a.norm = norm;
+    a.norm_prev = nullptr;
     a.first = 0;
-    float *cdev = (float *)(ws + L.cdev);
-    const dim3 grid((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kBY), (unsigned)div_up(d0, a.zc));
+    if (c < 0.f) M16_CUDA_TRY(cudaMemsetAsync(norm, 0xff, (size_t)nscales * 4, st));   // kNoNorm
     for (int s = 0; s < nscales; ++s) {
         AxisTaps tpx;
         const int rc = hessian_passes(img, d0, d1, d2, taps + (size_t)s * 9 * kMaxTaps, radius + 3 * s, ws, L, st, &tpx);
         if (rc != M16_OK) return rc;
         if (c >= 0.f) {
             a.first = s == 0;
-            launch_x_eig<true>(a, tpx, grid, st);
+            M16_CUDA_TRY(launch_x_eig<true>(a, tpx, st));
         } else {
             // scale s - 1's update rides along: its triple is read at each
             // voxel just before scale s's replaces it
-            a.c_prev = s > 0 ? cdev + s - 1 : nullptr;
+            a.norm = norm + s;
+            a.norm_prev = s > 0 ? norm + s - 1 : nullptr;
             a.first = s == 1;
-            launch_x_eig<false>(a, tpx, grid, st);
-            fr_c_kernel<<<1, 256, 0, st>>>(a.partials, L.nparts, cdev + s);
+            M16_CUDA_TRY(launch_x_eig<false>(a, tpx, st));
         }
-        M16_CUDA_TRY(cudaGetLastError());
     }
     if (c < 0.f) {
-        a.c_dev = cdev + nscales - 1;
-        a.c_prev = nullptr;
+        a.norm_prev = nullptr;
         a.first = nscales == 1;
         fr_update_kernel<<<blocks1d, 256, 0, st>>>(a, n);
         M16_CUDA_TRY(cudaGetLastError());
@@ -792,8 +875,10 @@ extern "C" int m16_frangi(const float *img, int32_t d0, int32_t d1, int32_t d2, 
         if (c >= 0.f) {
             for (int s = 0; s < nscales; ++s) c_used[s] = c;
         } else {
-            M16_CUDA_TRY(cudaMemcpyAsync(c_used, cdev, (size_t)nscales * 4, cudaMemcpyDeviceToHost, st));
+            std::vector<int> hn(nscales);
+            M16_CUDA_TRY(cudaMemcpyAsync(hn.data(), norm, (size_t)nscales * 4, cudaMemcpyDeviceToHost, st));
             M16_CUDA_TRY(cudaStreamSynchronize(st));
+            for (int s = 0; s < nscales; ++s) c_used[s] = scale_c(hn[s]);
         }
     }
     return M16_OK;
