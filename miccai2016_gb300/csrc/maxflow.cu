@@ -82,15 +82,25 @@ __global__ void mf_max_kernel(const float *__restrict__ img, int64_t n, float *_
     }
 }
 
-__global__ void mf_init_ctrl_kernel(const float *__restrict__ part, int nparts, int num_iter, MfCtrl *ctrl)
+__global__ void __launch_bounds__(256) mf_init_ctrl_kernel(const float *__restrict__ part, int nparts, int num_iter,
+                                                           MfCtrl *ctrl)
 {
-    if (threadIdx.x != 0) return;
+    __shared__ float sm[8];
+    __shared__ int snan;
+    if (threadIdx.x == 0) snan = 0;
+    __syncthreads();
     float m = -INFINITY;
-    bool nan = false;
-    for (int k = 0; k < nparts; ++k) {
+    for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
         const float v = part[k];
-        if (v != v) nan = true; else m = fmaxf(m, v);
+        if (v != v) snan = 1; else m = fmaxf(m, v);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, sm[w]);
+    const bool nan = snan != 0;
     ctrl->denom = (nan ? NAN : m) + FLT_MIN;   // np.max(img) + np.finfo(float32).tiny
     ctrl->stopped = 0;
     ctrl->iterations = num_iter;
@@ -362,7 +372,7 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
 
     const int init_blocks = (int)std::min<int64_t>(kMaxBlocks, div_up(n, 256));
     mf_max_kernel<<<init_blocks, 256, 0, st>>>(img, n, (float *)(ws + L.maxpart));
-    mf_init_ctrl_kernel<<<1, 32, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, ctrl);
+    mf_init_ctrl_kernel<<<1, 256, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, ctrl);
     const bool planar = metric == kMetricIso || metric == kMetricConst;
     mf_tile_init_kernel<<<init_blocks, 256, 0, st>>>(
         img, quat3, sqeigs, alpha, alpha_scalar, cs, ct, d2, (int64_t)d0 * d1, V.rcc, axis, ctrl,
@@ -523,7 +533,7 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
 
     const int init_blocks = (int)std::min<int64_t>(kMaxBlocks, div_up(n, 256));
     mf_max_kernel<<<init_blocks, 256, 0, st>>>(img, n, (float *)(ws + L.maxpart));
-    mf_init_ctrl_kernel<<<1, 32, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, a.ctrl);
+    mf_init_ctrl_kernel<<<1, 256, 0, st>>>((float *)(ws + L.maxpart), init_blocks, params->num_iter, a.ctrl);
     mf_init_kernel<<<init_blocks, 256, 0, st>>>(a, img, quat3, n);
     M16_CUDA_TRY(cudaGetLastError());
 

@@ -113,3 +113,29 @@ def test_a_small_workspace_takes_the_two_sweeps():
         torch.cuda.synchronize()
         assert np.array_equal(u.cpu().numpy().view(np.uint32), u_two.view(np.uint32))
         assert np.max(np.abs(u_tiles - u_two)) <= U_TOL
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 3), (5, 17, 33), (64, 64, 64), (90, 120, 140)])   # 1 to 400 blocks
+def test_the_last_block_gives_the_residuals(shape):
+    """The block that arrives last sums the partials in a fixed order: the
+    same bits whatever iterations are checked, solve after solve."""
+    inp = _inputs(3, shape)
+    u1, c1 = _cut(inp, (1.0, E, E), 29, 1)
+    for update in (1, 2, 7):
+        u, c = _cut(inp, (1.0, E, E), 29, update)
+        assert np.array_equal(u.view(np.uint32), u1.view(np.uint32))
+        assert np.array_equal(np.asarray(c.last_residuals), np.asarray(c1.last_residuals)[::update])
+
+
+def test_the_maximum_of_many_partials():
+    """The image's maximum in the last voxel, and a NaN image."""
+    shape = (50, 60, 70)
+    inp = _inputs(4, shape)
+    inp["img"][-1, -1, -1] = 50.0
+    u, _ = _cut(inp, (1.0, 1.0, 1.0), 4, 30)
+    ru, _, _ = O.maxflow_solve(inp["img"], inp["quats"], (1.0, 1.0, 1.0), inp["alpha"], inp["cs"], inp["ct"],
+                               num_iter=4, update=30, error_bound=-1.0)
+    assert np.max(np.abs(u - ru)) <= U_TOL
+    inp["img"][3, 4, 5] = np.nan
+    _, c = _cut(inp, (1.0, 1.0, 1.0), 4, 30)
+    assert c.last_iterations == 1 and np.isnan(c.last_residuals[0])   # the reference's check stops at NaN
