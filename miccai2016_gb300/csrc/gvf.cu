@@ -370,18 +370,23 @@ struct GvfTileLayout {
     int cap;
 };
 
+inline int gvf_iterations(bool resp) { return resp ? GvfShape<true>::K : GvfShape<false>::K; }
+inline int gvf_rows(bool resp) { return resp ? GvfShape<true>::Rows : GvfShape<false>::Rows; }
+inline int gvf_warps(bool resp) { return resp ? GvfShape<true>::NW : GvfShape<false>::NW; }
+
 // blocks of a launch of k iterations
 struct GvfTileGrid {
     int nx, ny, zc, blocks;
 };
 
-inline GvfTileGrid gvf_tile_grid(int d0, int d1, int d2, int k)
+inline GvfTileGrid gvf_tile_grid(int d0, int d1, int d2, int k, bool resp)
 {
-    const int ow = kTileLanes - 2 * gvf_halo(k), oh = kGvfRows - 2 * (k - 1);
+    const int rows = gvf_rows(resp), ow = kTileLanes - 2 * gvf_halo(k), oh = rows - 2 * (k - 1);
     GvfTileGrid G;
     G.nx = d2 <= kTileLanes ? 1 : (int)div_up(d2 - kTileLanes, ow) + 1;
-    G.ny = d1 <= kGvfRows ? 1 : (int)div_up(d1 - kGvfRows, oh) + 1;
-    const int64_t tiles = (int64_t)G.nx * G.ny, slots = (int64_t)kGvfBlocks * kSMs;
+    G.ny = d1 <= rows ? 1 : (int)div_up(d1 - rows, oh) + 1;
+    const int64_t tiles = (int64_t)G.nx * G.ny;
+    const int64_t slots = (int64_t)(resp ? GvfShape<true>::Blocks : GvfShape<false>::Blocks) * kSMs;
     // least waves x marched planes (2 k + 1 of them beyond the block's own)
     int64_t cost = INT64_MAX;
     G.zc = 1;
@@ -410,7 +415,8 @@ inline GvfTileLayout gvf_tile_layout(int d0, int d1, int d2, int has_response, i
     L.v = take(3 * np * 4);
     L.r = has_response ? take(np * 4) : 0;
     for (int b = 0; b < 2; ++b) L.g[b] = take(3 * np * 4);
-    for (int k = 1; k <= kGvfK; ++k) parts = std::max(parts, (size_t)k * gvf_tile_grid(d0, d1, d2, k).blocks);
+    for (int k = 1; k <= gvf_iterations(has_response != 0); ++k)
+        parts = std::max(parts, (size_t)k * gvf_tile_grid(d0, d1, d2, k, has_response != 0).blocks);
     L.partials = take(parts * 4);
     L.ctrl = take(sizeof(GvfCtrl));
     L.mags = take((size_t)L.cap * 8);
@@ -436,12 +442,12 @@ GvfTileKernel gvf_kernel_of(bool check, bool flat)
     return flat ? gvf_tile_kernel<K, RESP, false, true> : gvf_tile_kernel<K, RESP, false, false>;
 }
 
-template <int K>
-GvfTileKernel gvf_kernel(int k, bool resp, bool check, bool flat, size_t *smem)
+template <int K, bool RESP>
+GvfTileKernel gvf_kernel(int k, bool check, bool flat, size_t *smem)
 {
-    if (k < K) return gvf_kernel<(K > 1 ? K - 1 : 1)>(k, resp, check, flat, smem);
-    *smem = resp ? sizeof(GvfMem<K, true>) : sizeof(GvfMem<K, false>);
-    return resp ? gvf_kernel_of<K, true>(check, flat) : gvf_kernel_of<K, false>(check, flat);
+    if (k < K) return gvf_kernel<(K > 1 ? K - 1 : 1), RESP>(k, check, flat, smem);
+    *smem = sizeof(GvfMem<K, RESP>);
+    return gvf_kernel_of<K, RESP>(check, flat);
 }
 
 int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2, const double *voxel_size, double mu,
@@ -450,6 +456,8 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
                   const GvfTileLayout &L, char *ws, cudaStream_t st)
 {
     const int64_t n = (int64_t)d0 * d1 * d2, rows = (int64_t)d0 * d1;
+    const bool resp = response != nullptr;
+    const int pass = gvf_iterations(resp), tile_rows = gvf_rows(resp);
     GvfCtrl *ctrl = (GvfCtrl *)(ws + L.ctrl);
     double *mlog = (double *)(ws + L.mags);
     float *g[2] = {(float *)(ws + L.g[0]), (float *)(ws + L.g[1])};
@@ -476,22 +484,23 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
     a.partials = (float *)(ws + L.partials);
     a.err = &ctrl->error;
     CUtensorMap mg[2];
-    bool ok = gvf_map(&a.mv, ws + L.v, d0, d1, a.pitch, kGvfVW, kGvfRows);
-    for (int b = 0; b < 2; ++b) ok = ok && gvf_map(&mg[b], g[b], d0, d1, a.pitch, kGvfGW, kGvfRows + 2);
+    bool ok = gvf_map(&a.mv, ws + L.v, d0, d1, a.pitch, kGvfVW, tile_rows);
+    for (int b = 0; b < 2; ++b) ok = ok && gvf_map(&mg[b], g[b], d0, d1, a.pitch, kGvfGW, tile_rows + 2);
     if (response) {
         const cuuint64_t dims[3] = {(cuuint64_t)a.pitch, (cuuint64_t)d1, (cuuint64_t)d0};
         const cuuint64_t row = (cuuint64_t)a.pitch * 4, strides[2] = {row, row * d1};
-        const cuuint32_t box[3] = {kGvfVW, kGvfRows, 1};
+        const cuuint32_t box[3] = {kGvfVW, (cuuint32_t)tile_rows, 1};
         ok = ok && tile_map_encode(&a.mr, ws + L.r, 3, dims, strides, box);
     }
     if (!ok) return M16_ERR_CUDA;
-    GvfTileKernel kernels[kGvfK + 1][2];
-    size_t smem[kGvfK + 1];
-    GvfTileGrid grids[kGvfK + 1];
-    for (int k = 1; k <= kGvfK; ++k) {
-        grids[k] = gvf_tile_grid(d0, d1, d2, k);
+    GvfTileKernel kernels[kGvfMaxK + 1][2];
+    size_t smem[kGvfMaxK + 1];
+    GvfTileGrid grids[kGvfMaxK + 1];
+    for (int k = 1; k <= pass; ++k) {
+        grids[k] = gvf_tile_grid(d0, d1, d2, k, resp);
         for (int c = 0; c < 2; ++c) {
-            kernels[k][c] = gvf_kernel<kGvfK>(k, response != nullptr, c != 0, d1 < kGvfRows, &smem[k]);
+            kernels[k][c] = resp ? gvf_kernel<GvfShape<true>::K, true>(k, c != 0, d1 < tile_rows, &smem[k])
+                                 : gvf_kernel<GvfShape<false>::K, false>(k, c != 0, d1 < tile_rows, &smem[k]);
             M16_CUDA_TRY(
                 cudaFuncSetAttribute(kernels[k][c], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[k]));
         }
@@ -508,7 +517,7 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
         s.checks = 0;
         if (!always)
             for (int j = 0; j < k; ++j) s.checks |= (it + j) % update == 0 ? 1 << j : 0;
-        cudaError_t e = launch_pdl_smem(kernels[k][s.checks != 0], dim3(G.blocks), dim3(kTileLanes, kGvfNW), smem[k], st, true, s);
+        cudaError_t e = launch_pdl_smem(kernels[k][s.checks != 0], dim3(G.blocks), dim3(kTileLanes, gvf_warps(resp)), smem[k], st, true, s);
         if (e == cudaSuccess && s.checks)
             e = launch_pdl(gvf_tile_check_kernel, dim3(1), dim3(256), st, true, (const float *)a.partials, G.blocks,
                            1.0 / (double)n, tol, it, k, update, L.cap, ctrl, mlog);
@@ -518,7 +527,7 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
     // previous one (which reads the buffer it writes) before any access
     int sweeps = 0;
     for (int done = 0; done < n_iters; ++sweeps) {
-        const int k = std::min(kGvfK, n_iters - done);
+        const int k = std::min(pass, n_iters - done);
         M16_CUDA_TRY(sweep(first_iter + done, k, (buf0 + sweeps) & 1, false));
         done += k;
     }
@@ -530,11 +539,11 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
     int buf = buf0;
     if (!was_stopped) {
         const int ran = done - first_iter;
-        buf = (buf0 + (int)div_up(ran, kGvfK)) & 1;
+        buf = (buf0 + (int)div_up(ran, pass)) & 1;
         // stopped inside a sweep: its iterations up to there again, from the
         // buffer it read
-        if (h.stopped && ran % kGvfK && ran < n_iters)
-            M16_CUDA_TRY(sweep(done - ran % kGvfK, ran % kGvfK, 1 - buf, true));
+        if (h.stopped && ran % pass && ran < n_iters)
+            M16_CUDA_TRY(sweep(done - ran % pass, ran % pass, 1 - buf, true));
     }
     gvf_tile_output_kernel<<<blocks1d, 256, 0, st>>>(g[buf], d2, rows, normalize, buf, ctrl, g3);
     M16_CUDA_TRY(cudaGetLastError());

@@ -3,7 +3,7 @@
 //
 // Fields are planar and padded (tile_pitch), the components one behind the
 // other, so that one tensor copy brings all three.  A block marches along z
-// with 32 columns and kGvfRows rows; stage k (the k-th iteration) works a plane
+// with 32 columns and GvfShape::Rows rows; stage k (the k-th iteration) works a plane
 // behind stage k - 1.  A lane keeps kGvfRT rows of two adjacent columns
 // (f32x2.cuh), half a warp a row, three planes of each stage's input in
 // registers.  Stage 1 reads the x and y neighbours of its plane from the copied
@@ -12,14 +12,20 @@
 // rows stored a step before, so one barrier a step is enough.  A block writes
 // all but K - 1 rows (and as many columns, rounded up to a pair) on each side.
 //
-// Bound: 36 bytes a voxel for K iterations, and about 66 instructions a computed
-// voxel and iteration.  Measured on GB300 at 256^3 (100 iterations, set-up and
-// output included): one iteration a pass over 40 bytes 124 us an iteration; K =
-// 1 here 94, K = 2 66 (0.72 of the copy rate, issue 54 %, shared memory 60 %
-// busy), K = 3 73 (its slots leave one block per SM); K = 2 with scalar
-// arithmetic 76.  2 x 12 half-warps of rows, 2 blocks per SM; 16 rows and 3
-// blocks 66, 32 rows and one block 79, one row a lane 93, four rows 109
-// (spills).  75 x 93 x 110, 300 iterations with a response: 10.1 -> 8.1.
+// Bound: 36 bytes a voxel for K iterations (40 with a response), and about 66
+// instructions a computed voxel and iteration.  Measured on GB300 at 256^3 (100
+// iterations, set-up and output included): one iteration a pass over 40 bytes
+// 124 us an iteration; K = 1 here 94, K = 2 66 (0.72 of the copy rate, issue 54
+// %, shared memory 60 % busy), K = 3 73 (its slots leave one block per SM); K =
+// 2 with scalar arithmetic 76.  2 x 12 half-warps of rows, 2 blocks per SM; 16
+// rows and 3 blocks 66, 32 rows and one block 79, one row a lane 93, four rows
+// 109 (spills).
+//
+// With a response that shape's slots fill more than half of an SM's shared
+// memory, so one block of six warps ran on each (256^3 102 us an iteration, 97 x
+// 161 x 203 27.2, 75 x 93 x 110 8.2).  There one block of 8 warps (32 rows) and K
+// = 3 take 73, 17.5 and 6.3; two blocks of 20 rows and K = 2 82, 18.3 and 6.7; of
+// 16 rows 80, 19.0 and 6.3.
 #pragma once
 
 #include "common.cuh"
@@ -29,22 +35,14 @@
 namespace m16 {
 namespace {
 
-#ifndef M16_GVF_K
-#define M16_GVF_K 2
-#endif
-#ifndef M16_GVF_RT
-#define M16_GVF_RT 2
-#endif
-#ifndef M16_GVF_NW
-#define M16_GVF_NW 6
-#endif
-#ifndef M16_GVF_BLOCKS
-#define M16_GVF_BLOCKS 2
-#endif
-constexpr int kGvfK = M16_GVF_K;
-constexpr int kGvfRT = M16_GVF_RT, kGvfNW = M16_GVF_NW, kGvfBlocks = M16_GVF_BLOCKS;
-constexpr int kGvfGroups = 2 * kGvfNW;               // half-warps
-constexpr int kGvfRows = kGvfRT * kGvfGroups;
+constexpr int kGvfRT = 2;                            // rows per lane
+// iterations of a pass, warps of a block and blocks per SM
+template <bool RESP>
+struct GvfShape {
+    static constexpr int K = RESP ? 3 : 2, NW = RESP ? 8 : 6, Blocks = RESP ? 1 : 2;
+    static constexpr int Groups = 2 * NW, Rows = kGvfRT * Groups;   // half-warps, rows of a block
+};
+constexpr int kGvfMaxK = 3;
 constexpr int kGvfGW = 40, kGvfVW = 32;              // copied row lengths
 // columns a block leaves out on each inner side: K - 1, pairs of them, with
 // starts on a 16-byte boundary
@@ -65,14 +63,14 @@ struct GvfTileArgs {
 
 template <int K, bool RESP>
 struct GvfMem {
-    static constexpr int H = kGvfRows, Lag = K < 2 ? 2 : K, S = Lag + 2;
+    static constexpr int H = GvfShape<RESP>::Rows, Lag = K < 2 ? 2 : K, S = Lag + 2;
     struct Slot {   // v of plane p, g of plane p + 1
         alignas(128) float g[3][H + 2][kGvfGW];
         alignas(128) float v[3][H][kGvfVW];
         alignas(128) float r[RESP ? H : 1][kGvfVW];
     } slot[S];
     // [stage][step parity][half-warp][first, last row] of each later stage's input
-    f2 edge[K > 1 ? K - 1 : 1][2][kGvfGroups + 2][2][3][16];
+    f2 edge[K > 1 ? K - 1 : 1][2][GvfShape<RESP>::Groups + 2][2][3][16];
     uint64_t full[S];
 };
 
@@ -87,13 +85,14 @@ __device__ __forceinline__ void gvf_copy(void *dst, const CUtensorMap *map, int 
 // FLAT: fewer rows than a block has, so that the last row of the volume may be
 // any row of a lane; otherwise the last tile ends on it.
 template <int K, bool RESP, bool CHECK, bool FLAT>
-__global__ void __launch_bounds__(kTileLanes *kGvfNW, kGvfBlocks) gvf_tile_kernel(const __grid_constant__ GvfTileArgs a)
+__global__ void __launch_bounds__(kTileLanes *GvfShape<RESP>::NW, GvfShape<RESP>::Blocks)
+    gvf_tile_kernel(const __grid_constant__ GvfTileArgs a)
 {
     extern __shared__ __align__(128) unsigned char gvf_mem[];
     __shared__ float red[32];
     typedef GvfMem<K, RESP> Mem;
     Mem &M = *reinterpret_cast<Mem *>(gvf_mem);
-    constexpr int RT = kGvfRT, H = kGvfRows, S = Mem::S, Lag = Mem::Lag;
+    constexpr int RT = kGvfRT, H = Mem::H, S = Mem::S, Lag = Mem::Lag;
     const int lane = threadIdx.x, warp = threadIdx.y;
     const bool copier = lane == 0 && warp == 0;
     if (copier) {

@@ -65,3 +65,32 @@ def test_pieces_give_the_bits_of_the_whole():
     assert [i for i, _ in seen] == [0, 4, 8, 12, 16, 20]
     assert np.array_equal(g.view(np.uint32), h.view(np.uint32))
     assert obj.last_iterations == whole.last_iterations == 23
+
+
+# with a response a block has 32 rows and three iterations a pass
+@pytest.mark.parametrize("shape", [(3, 31, 31), (1, 32, 32), (7, 33, 33), (5, 60, 60), (2, 61, 61), (70, 89, 3)])
+def test_edges_with_a_response(shape):
+    v = _field(sum(shape), shape)
+    r = np.random.RandomState(3).uniform(0, 1, shape).astype(np.float32)
+    for maxiter in (1, 2, 3, 4, 5, 13):
+        g, obj = _gvf(v, maxiter, 4, response=r)
+        ref, _, mags = O.gvf_run(v, 0.2, maxiter, 4, response=r)
+        assert np.max(np.abs(g - ref)) <= 1e-4 * max(float(np.max(np.abs(ref))), 1e-6), maxiter
+        np.testing.assert_allclose(obj.last_mags, mags[:len(obj.last_mags)], rtol=1e-4, atol=1e-9)
+
+
+@pytest.mark.parametrize("update", [1, 2, 3, 4])
+def test_stops_and_pieces_with_a_response(update):
+    """The response that is taken without one, |v|^2, given as a field."""
+    v = (np.float32([0.5, 0.4, 0.3]) + 0.1 * _field(9, (20, 41, 50))).astype(np.float32)
+    r = np.sum(v.astype(np.float64) ** 2, -1).astype(np.float32)
+    whole, full = _gvf(v, 20, update, response=r)
+    m = full.last_mags
+    assert np.all(np.diff(m) < 0)
+    for k in range(1, len(m)):
+        g, obj = _gvf(v, 20, update, tol=float(0.5 * (m[k] + m[k - 1])), response=r)
+        assert obj.last_iterations == k * update + 1
+        h, _ = _gvf(v, obj.last_iterations, update, response=r)
+        assert np.array_equal(g.view(np.uint32), h.view(np.uint32)), k
+    p, _ = _gvf(v, 20, update, response=r, callback=lambda f, i, mag: None)
+    assert np.array_equal(p.view(np.uint32), whole.view(np.uint32))
