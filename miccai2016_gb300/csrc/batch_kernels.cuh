@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) bt_tile_kern
     const int nx = T.nx, ny = T.ny, zc = T.zc;
     const int bx = wk.y % nx, t = wk.y / nx, by = t % ny, za = t / ny * zc;
     float acc[2] = {0.f, 0.f};
-    tile_sweep<K, METRIC, ASRC, true, false, CHECK>(V, M, bx, by, za, min(za + zc, V.d0), acc);
+    tile_sweep<K, METRIC, ASRC, true, false, CHECK>(V, M, bx, by, za, min(za + zc, V.d0), acc, [] {}, nullptr);
     if (CHECK) {
         const float sum = block_sum(acc[K - 1], red);
         if (threadIdx.x == 0 && threadIdx.y == 0) partials[T.part_off + wk.y] = sum;

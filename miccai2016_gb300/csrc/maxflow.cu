@@ -395,17 +395,18 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
         pool.reset(new EventPool(std::min(num_iter, chunk) + 2));
         if (!pool->ok) return M16_ERR_CUDA;
     }
+    int it = 0;
     auto sweep = [&](int count, bool check, int buf, bool always) -> cudaError_t {
         const MfTileLaunch &K = kernels[count - 1][check];
         MfTileArgs a = args[buf];
         if (always) a.stopped = nullptr;
-        return launch_pdl_smem(K.kernel, dim3(L.nblocks), dim3(kTileLanes, kTileNW), K.smem, st, pdl, a);
+        // the first one reads what the set-up kernel wrote before it waits: not early
+        return launch_pdl_smem(K.kernel, dim3(L.nblocks), dim3(kTileLanes, kTileNW), K.smem, st, pdl && it > 0, a);
     };
     int pair_n = 0;
     double pair_ms = 0.0;
     MfCtrl hctrl;
     hctrl.stopped = 0;
-    int it = 0;
     while (it < num_iter) {
         const int end = std::min(num_iter, it + chunk), begin = it;
         int slots = 0;

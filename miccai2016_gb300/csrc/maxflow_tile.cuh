@@ -28,15 +28,16 @@ __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) mf_tile_kern
     __shared__ float red[32];
     TileMem<METRIC, ASRC> &M = *reinterpret_cast<TileMem<METRIC, ASRC> *>(tile_mem);
     tile_init(M);
-    pdl_wait();
-    pdl_launch_next();
-    if (a.stopped && __ldcg(a.stopped)) return;
     TileView V = a.V;
     V.mh = &a.mh; V.mu = &a.mu; V.mdir = &a.mdir; V.meig = &a.meig; V.mcaps = &a.mcaps; V.mrad = &a.mrad;
     const int bx = blockIdx.x % a.nx, t = blockIdx.x / a.nx;
     const int by = t % a.ny, za = t / a.ny * a.zc;
     float acc[2] = {0.f, 0.f};
-    tile_sweep<K, METRIC, ASRC, false, SUP, CHECK>(V, M, bx, by, za, min(za + a.zc, V.d0), acc);
+    const bool ran = tile_sweep<K, METRIC, ASRC, false, SUP, CHECK>(V, M, bx, by, za, min(za + a.zc, V.d0), acc, [] {
+        pdl_wait();
+        pdl_launch_next();
+    }, a.stopped);
+    if (!ran) return;
     if (CHECK) {
         const float s0 = block_sum(acc[0], red);
         __syncthreads();
