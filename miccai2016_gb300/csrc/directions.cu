@@ -591,6 +591,95 @@ __global__ void __launch_bounds__(kBX * kBY) dr_adjust_indexed_kernel(
     }
 }
 
+// The same for few ridge points: no cells.  A block takes 8 x 8 x 8 voxels and
+// looks at every point twice: the least of the points' greatest distances to the
+// block bounds every voxel's nearest distance, and only points whose least
+// distance to the block is not above it are compared with the voxels.  Distances
+// to the block take per axis the least and the greatest |p - q| over its voxels;
+// every step of ref_dist is monotone, rounding included, so the bounds hold for
+// the rounded distances and the result is the exact search's, ties included.
+//
+// Bound by issue: about R / 8 instructions a warp for the two looks and a dozen
+// for every candidate.  Measured on ridge-like curves, the cells' search against
+// this one: 128^3, 770 points 456 -> 69 us, 8000 429 -> 205, 16000 468 -> 347; 256^3,
+// 2000 points 4341 -> 598, 8000 4132 -> 1267, 16000 4096 -> 2103, 60000 3581
+// against 6566; 64^3, 770 points 88 -> 24, 8000 89 -> 77, 16000 95 against 127.
+// The two looks grow with R while denser points leave the cells less to search:
+// this kernel takes up to kFewPoints points, and no more than one per kFewVoxels.
+constexpr int kFewTile = 8;
+constexpr int64_t kFewPoints = 16384, kFewVoxels = 32;
+
+__global__ void __launch_bounds__(256) dr_adjust_few_kernel(float *__restrict__ dirs3,
+                                                            const uint16_t *__restrict__ coords,
+                                                            const float *__restrict__ rdirs, int R, int d0, int d1,
+                                                            int d2, int nx, int ny, float s0, float s1, float s2)
+{
+    __shared__ float4 list[256];
+    __shared__ float red[8];
+    __shared__ int count[2];
+    const int t = threadIdx.x;
+    const int x0 = (int)(blockIdx.x % nx) * kFewTile, q = blockIdx.x / nx;
+    const int y0 = q % ny * kFewTile, z0 = q / ny * kFewTile;
+    const int x1 = min(x0 + kFewTile, d2) - 1, y1 = min(y0 + kFewTile, d1) - 1, z1 = min(z0 + kFewTile, d0) - 1;
+    const int x = x0 + (t & 7), y = y0 + (t >> 3 & 7), z = z0 + (t >> 6);   // and z + 4
+    auto far_gap = [](int p, int lo, int hi, float s) { return __fmul_rn((float)max(abs(p - lo), abs(p - hi)), s); };
+    float bound = INFINITY;
+    for (int j = t; j < R; j += 256) {
+        const int a = coords[3 * j], b = coords[3 * j + 1], c = coords[3 * j + 2];
+        bound = fminf(bound, ref_dist(far_gap(a, z0, z1, s0), far_gap(b, y0, y1, s1), far_gap(c, x0, x1, s2)));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bound = fminf(bound, __shfl_xor_sync(0xffffffffu, bound, o));
+    if ((t & 31) == 0) red[t >> 5] = bound;
+    if (t < 2) count[t] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) bound = fminf(bound, red[w]);
+
+    const float px = (float)x, py = (float)y, pz[2] = {(float)z, (float)(z + 4)};
+    float best[2] = {INFINITY, INFINITY};
+    int bj[2] = {INT_MAX, INT_MAX};
+    for (int j0 = 0, round = 0; j0 < R; j0 += 256, round ^= 1) {
+        const int j = j0 + t;
+        if (j < R) {
+            const int a = coords[3 * j], b = coords[3 * j + 1], c = coords[3 * j + 2];
+            if (!(ref_dist(axis_gap(a, z0, z1, s0), axis_gap(b, y0, y1, s1), axis_gap(c, x0, x1, s2)) > bound))
+                list[atomicAdd(&count[round], 1)] = make_float4((float)a, (float)b, (float)c, __int_as_float(j));
+        }
+        __syncthreads();
+        const int n = count[round];
+        if (t == 0) count[round ^ 1] = 0;   // last read before the barrier of the round before's end
+        for (int k = 0; k < n; ++k) {
+            const float4 p = list[k];
+            const int jk = __float_as_int(p.w);
+            const float f1 = __fmul_rn(fabsf(__fsub_rn(py, p.y)), s1), f2 = __fmul_rn(fabsf(__fsub_rn(px, p.z)), s2);
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const float d = ref_dist(__fmul_rn(fabsf(__fsub_rn(pz[v], p.x)), s0), f1, f2);
+                if (d < best[v] || (d == best[v] && jk < bj[v])) {
+                    best[v] = d;
+                    bj[v] = jk;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (x >= d2 || y >= d1) return;
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        if (z + 4 * v >= d0 || bj[v] == INT_MAX) continue;
+        float *dir = dirs3 + 3 * (((int64_t)(z + 4 * v) * d1 + y) * d2 + x);
+        const float w0 = __ldg(rdirs + 3 * (int64_t)bj[v]), w1 = __ldg(rdirs + 3 * (int64_t)bj[v] + 1),
+                    w2 = __ldg(rdirs + 3 * (int64_t)bj[v] + 2);
+        const float dot = __fadd_rn(__fadd_rn(__fmul_rn(dir[0], w0), __fmul_rn(dir[1], w1)), __fmul_rn(dir[2], w2));
+        if (dot < 0.f) {
+            dir[0] = -dir[0];
+            dir[1] = -dir[1];
+            dir[2] = -dir[2];
+        }
+    }
+}
+
 inline int blocks1d(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(16 * kSMs, div_up(n, 256))); }
 
 }  // namespace
@@ -689,6 +778,14 @@ extern "C" int m16_adjust_nonridge_signs_indexed(float *dirs3, int32_t d0, int32
     const NrLayout L = nr_layout(g, num_ridge);
     if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255)) return M16_ERR_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
+    const int64_t fx = div_up(d2, kFewTile), fy = div_up(d1, kFewTile), fb = fx * fy * div_up(d0, kFewTile);
+    if (num_ridge <= std::min(kFewPoints, (int64_t)d0 * d1 * d2 / kFewVoxels) && fb <= INT32_MAX) {
+        dr_adjust_few_kernel<<<(unsigned)fb, 256, 0, st>>>(dirs3, coords, rdirs, (int)num_ridge, d0, d1, d2, (int)fx,
+                                                           (int)fy, (float)scaling3[0], (float)scaling3[1],
+                                                           (float)scaling3[2]);
+        M16_CUDA_TRY(cudaGetLastError());
+        return M16_OK;
+    }
     char *ws = (char *)workspace;
     unsigned *count = (unsigned *)(ws + L.count), *start = (unsigned *)(ws + L.start), *bsum = (unsigned *)(ws + L.bsum);
     float4 *pts = (float4 *)(ws + L.pts);
