@@ -22,7 +22,8 @@ def _filter(sigma, c):
 
 # radius round(4 sigma): 1, 2, 3, 4, 12, 15, 16 (instantiated), 17, 18, 63 (any)
 @pytest.mark.parametrize("sigma", [0.25, 0.5, 0.75, 1.0, 3.0, 3.75, 4.0, 4.25, 4.5, 15.75])
-@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 9, 31), (2, 8, 128), (4, 3, 129), (2, 17, 257)])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 9, 31), (2, 5, 32), (2, 4, 33), (2, 8, 128), (4, 3, 129), (1, 6, 160),
+                                   (1, 6, 161), (2, 17, 257)])
 def test_x_pass_equals_the_plain_kernels(shape, sigma):
     from miccai2016_gb300.qfrangi_gpu import eigendecomposition, hessian
     rng = np.random.RandomState(shape[2] + int(100 * sigma))
