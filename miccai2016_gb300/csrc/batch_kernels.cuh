@@ -27,10 +27,11 @@
 // so captured launches can be replayed.
 //
 // Measured on GB300: 16 grid points at 128^3, anisotropic and isotropic (32
-// instances), 358 -> 154 ms against groups of four interleaved instances in a
-// flow and a label launch per iteration; eight uneven volumes 46.4 -> 21.6 ms;
-// ten served requests 112 -> 51.6 ms.  Bound by HBM: 48 bytes of state per
-// voxel and two iterations (tile_sweep.cuh).
+// instances), 358 -> 152 ms against groups of four interleaved instances in a
+// flow and a label launch per iteration; eight uneven volumes 39.6 -> 18.5 ms;
+// ten served requests 113 -> 51 ms.  Bound by HBM where the tiles fit the
+// volume (48 bytes of state per voxel and two iterations), by the march's
+// instructions on the halo where they do not (128^3: 1.56 times the voxels).
 //
 // The compact sweeps at the end (one buffer, planar fields, a flow and a label
 // launch per iteration) take the instances whose double-buffered state does

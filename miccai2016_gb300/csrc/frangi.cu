@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(kBX * kBY) fr_conv_y_run_kernel(const float *_
 // wavefront per 32 columns each: 272 us of the radius-12 pass at 256^3 at one
 // wavefront a clock, which the eigensolve did not hide; four columns per lane
 // read 6 (2R + 4) / 4.  Measured at 256^3, radius 12 / 8 / 4: 752 / 699 / 577 us ->
-// 714 / 670 / 541 us; at 45 x 61 x 83, radius 18: 46 -> 24 us.
+// 714 / 670 / 541 us (blocks of eight warps); at 45 x 61 x 83, radius 18: 46 -> 24.
 //
 // The Jacobi's data-dependent sweep count makes a warp wait for its slowest
 // voxel (77 % of the lanes' sweeps are of use).  Handing each lane the next
