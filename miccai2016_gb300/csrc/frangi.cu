@@ -55,7 +55,7 @@ __device__ __forceinline__ int mirror(int p, int n)
 // and every tap too.  Each output accumulates its taps in the order j = 0..K-1
 // (tap K-1-j), as the specialised passes do.  Bound by latency and issue on a
 // small volume: at 45 x 61 x 83, radius 18 and 24, the y passes with one output
-// per thread took 44 us each, every tap waiting for its loads, and 30 us so.
+// per thread took 44 us each, every tap waiting for its loads.
 constexpr int kAnyRun = 4, kAnyTaps = 8;
 constexpr int kAnyBY = 4;   // rows of a block: small volumes have few threads, and smaller blocks spread them
 
@@ -73,14 +73,15 @@ __device__ __forceinline__ void any_load(const float *__restrict__ col, int64_t 
 }
 
 // acc[o] += t[jj] * v[o + jj] over the block's taps in order
-__device__ __forceinline__ void any_fma(const float (&t)[kAnyTaps], int nt, const float (&v)[kAnyRun + kAnyTaps - 1],
-                                        float (&acc)[kAnyRun])
+template <int RUN>
+__device__ __forceinline__ void any_fma(const float (&t)[kAnyTaps], int nt, const float (&v)[RUN + kAnyTaps - 1],
+                                        float (&acc)[RUN])
 {
 #pragma unroll
     for (int jj = 0; jj < kAnyTaps; ++jj)
         if (jj < nt)
 #pragma unroll
-            for (int o = 0; o < kAnyRun; ++o) acc[o] = fmaf(t[jj], v[o + jj], acc[o]);
+            for (int o = 0; o < RUN; ++o) acc[o] = fmaf(t[jj], v[o + jj], acc[o]);
 }
 
 __device__ __forceinline__ void any_taps(const AxisTaps &tp, int order, int j0, int K, float (&t)[kAnyTaps])
@@ -109,7 +110,7 @@ __global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_z_kernel(const float *__
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 any_taps(tp, k, j0, K, t);
-                any_fma(t, K - j0, v, acc[k]);
+                any_fma<kAnyRun>(t, K - j0, v, acc[k]);
             }
         }
 #pragma unroll
@@ -124,50 +125,80 @@ __global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_z_kernel(const float *__
     }
 }
 
-// pass 2: y (axis 1), the six products; block row = kAnyRun rows of the volume
-__global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_y_kernel(const float *__restrict__ z0,
-                                                                 const float *__restrict__ z1,
-                                                                 const float *__restrict__ z2, float *__restrict__ six,
-                                                                 int d0, int d1, int d2,
-                                                                 const __grid_constant__ AxisTaps tp)
+// pass 2: y (axis 1), the six products.  A block takes 32 columns and kAnyRows
+// rows of a plane, puts them with their mirrored halo into shared memory, and
+// every warp computes kRun rows from there.  Reading the inputs anew for every
+// run of four rows, each address mirrored again (a volume of 61 rows has hardly a
+// run with all of 49 taps inside), took 28 us at 45 x 61 x 83, radius 18 and 24;
+// this 14.  Whole filters: 120 x 120 x 100, scales 2 to 6, 514 -> 458 us; 200^3,
+// scales 4.5 and 6, 2315 -> 1990; 30 x 300 x 40, radii 18 and 40, 264 -> 204.
+constexpr int kAnyRows = 64, kAnyOut = 8;   // rows of a block and of a warp
+static_assert(kAnyRows == kAnyOut * kBY, "a run of rows per warp");
+
+constexpr size_t fr_any_y_bytes(int r) { return sizeof(float) * 3 * (kAnyRows + 2 * r) * kBX; }
+
+__global__ void __launch_bounds__(kBX * kBY) fr_conv_y_kernel(const float *__restrict__ z0,
+                                                              const float *__restrict__ z1,
+                                                              const float *__restrict__ z2, float *__restrict__ six,
+                                                              int d0, int d1, int d2,
+                                                              const __grid_constant__ AxisTaps tp)
 {
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int ya = (blockIdx.y * kAnyBY + threadIdx.y) * kAnyRun;
-    if (x >= d2 || ya >= d1) return;
+    extern __shared__ __align__(16) float any_rows[];
+    const int lane = threadIdx.x, warp = threadIdx.y;
+    const int x = blockIdx.x * kBX + lane, xc = min(x, d2 - 1);
+    const int y0 = blockIdx.y * kAnyRows, ya = y0 + warp * kAnyOut;
     const int64_t s0 = (int64_t)d1 * d2, n = s0 * d0;
     const int r = tp.radius, K = 2 * r + 1;
-    const bool inner = ya - r >= 0 && ya + kAnyRun - 1 + r < d1;
+    const int rows = min(kAnyRows, d1 - y0) + 2 * r, part = (kAnyRows + 2 * r) * kBX;
     for (int z = blockIdx.z; z < d0; z += gridDim.z) {
-        const int64_t plane = (int64_t)z * s0 + x;
-        float A[kAnyRun] = {}, B[kAnyRun] = {}, C[kAnyRun] = {}, D[kAnyRun] = {}, E[kAnyRun] = {}, F[kAnyRun] = {};
-        for (int j0 = 0; j0 < K; j0 += kAnyTaps) {
-            const int first = ya - r + j0, nt = K - j0;
-            float v0[kAnyRun + kAnyTaps - 1], v1[kAnyRun + kAnyTaps - 1], v2[kAnyRun + kAnyTaps - 1], t[kAnyTaps];
-            any_load(z0 + plane, d2, first, d1, inner, v0);
-            any_load(z1 + plane, d2, first, d1, inner, v1);
-            any_load(z2 + plane, d2, first, d1, inner, v2);
-            any_taps(tp, 0, j0, K, t);
-            any_fma(t, nt, v2, A);   // A = y0 Z2
-            any_fma(t, nt, v0, C);   // C = y0 Z0
-            any_fma(t, nt, v1, E);   // E = y0 Z1
-            any_taps(tp, 1, j0, K, t);
-            any_fma(t, nt, v1, D);   // D = y1 Z1
-            any_fma(t, nt, v0, F);   // F = y1 Z0
-            any_taps(tp, 2, j0, K, t);
-            any_fma(t, nt, v0, B);   // B = y2 Z0
+        const int64_t plane = (int64_t)z * s0 + xc;
+        for (int k = warp; k < rows; k += kBY) {
+            const int64_t i = plane + (int64_t)mirror(y0 - r + k, d1) * d2;
+            float *q = any_rows + k * kBX + lane;
+            q[0] = __ldg(z0 + i);
+            q[part] = __ldg(z1 + i);
+            q[2 * part] = __ldg(z2 + i);
         }
+        __syncthreads();
+        if (ya < d1) {
+            float A[kAnyOut] = {}, B[kAnyOut] = {}, C[kAnyOut] = {}, D[kAnyOut] = {}, E[kAnyOut] = {}, F[kAnyOut] = {};
+            for (int j0 = 0; j0 < K; j0 += kAnyTaps) {
+                // rows past the last one that an output needs are read where they exist
+                const int first = warp * kAnyOut + j0, nt = K - j0;
+                float v0[kAnyOut + kAnyTaps - 1], v1[kAnyOut + kAnyTaps - 1], v2[kAnyOut + kAnyTaps - 1], t[kAnyTaps];
 #pragma unroll
-        for (int o = 0; o < kAnyRun; ++o) {
-            if (ya + o < d1) {
-                const int64_t i = plane + (int64_t)(ya + o) * d2;
-                six[i] = A[o];
-                six[n + i] = B[o];
-                six[2 * n + i] = C[o];
-                six[3 * n + i] = D[o];
-                six[4 * n + i] = E[o];
-                six[5 * n + i] = F[o];
+                for (int p = 0; p < kAnyOut + kAnyTaps - 1; ++p) {
+                    const float *q = any_rows + min(first + p, rows - 1) * kBX + lane;
+                    v0[p] = q[0];
+                    v1[p] = q[part];
+                    v2[p] = q[2 * part];
+                }
+                any_taps(tp, 0, j0, K, t);
+                any_fma<kAnyOut>(t, nt, v2, A);   // A = y0 Z2
+                any_fma<kAnyOut>(t, nt, v0, C);   // C = y0 Z0
+                any_fma<kAnyOut>(t, nt, v1, E);   // E = y0 Z1
+                any_taps(tp, 1, j0, K, t);
+                any_fma<kAnyOut>(t, nt, v1, D);   // D = y1 Z1
+                any_fma<kAnyOut>(t, nt, v0, F);   // F = y1 Z0
+                any_taps(tp, 2, j0, K, t);
+                any_fma<kAnyOut>(t, nt, v0, B);   // B = y2 Z0
+            }
+            if (x < d2) {
+#pragma unroll
+                for (int o = 0; o < kAnyOut; ++o) {
+                    if (ya + o < d1) {
+                        const int64_t i = plane + (int64_t)(ya + o) * d2;
+                        six[i] = A[o];
+                        six[n + i] = B[o];
+                        six[2 * n + i] = C[o];
+                        six[3 * n + i] = D[o];
+                        six[4 * n + i] = E[o];
+                        six[5 * n + i] = F[o];
+                    }
+                }
             }
         }
+        __syncthreads();
     }
 }
 
@@ -711,6 +742,7 @@ __global__ void __launch_bounds__(kBX * kXBY) fr_conv_x_eig_kernel(const __grid_
     if (!FUSED_UPDATE) block_max_to_norm<kWarps>(mx, red, a.norm);
 }
 
+static_assert(kRunMaxR == 16, "the cases below");
 #define FR_RADIUS_CASES(CALL)                                                                                   \
     case 1: CALL(1); break;   case 2: CALL(2); break;   case 3: CALL(3); break;   case 4: CALL(4); break;     \
     case 5: CALL(5); break;   case 6: CALL(6); break;   case 7: CALL(7); break;   case 8: CALL(8); break;     \
@@ -844,15 +876,19 @@ int hessian_passes(const float *img, int d0, int d1, int d2, const float *taps, 
         default: fr_conv_z_kernel<<<any_z, block_any, 0, st>>>(img, z, z + n, z + 2 * n, d0, d1, d2, tpz); break;
     }
 #undef FR_Z_CALL
-    const dim3 any_y((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kAnyBY * kAnyRun),
-                     (unsigned)std::min(65535, d0));
+    const dim3 any_y((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kAnyRows), (unsigned)std::min(65535, d0));
+    const size_t any_y_bytes = fr_any_y_bytes(tpy.radius);
     // one z plane per block of the specialised y pass (grid z limit 65535)
     const dim3 grid_y((unsigned)div_up(d2, kBX), (unsigned)div_up(d1, kBY * kRun), (unsigned)d0);
     const int ry = d0 <= 65535 ? tpy.radius : 0;
 #define FR_Y_CALL(R) fr_conv_y_run_kernel<R><<<grid_y, block, 0, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, tpy)
     switch (ry) {
         FR_RADIUS_CASES(FR_Y_CALL)
-        default: fr_conv_y_kernel<<<any_y, block_any, 0, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, tpy); break;
+        default:
+            M16_CUDA_TRY(cudaFuncSetAttribute(fr_conv_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)fr_any_y_bytes((kMaxTaps - 1) / 2)));
+            fr_conv_y_kernel<<<any_y, block, any_y_bytes, st>>>(z, z + n, z + 2 * n, six, d0, d1, d2, tpy);
+            break;
     }
 #undef FR_Y_CALL
     M16_CUDA_TRY(cudaGetLastError());
