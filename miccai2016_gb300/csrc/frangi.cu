@@ -56,7 +56,7 @@ __device__ __forceinline__ int mirror(int p, int n)
 // (tap K-1-j), as the specialised passes do.  Bound by latency and issue on a
 // small volume: at 45 x 61 x 83, radius 18 and 24, the y passes with one output
 // per thread took 44 us each, every tap waiting for its loads.
-constexpr int kAnyRun = 4, kAnyTaps = 8;
+constexpr int kAnyRun = 8, kAnyTaps = 8;
 constexpr int kAnyBY = 4;   // rows of a block: small volumes have few threads, and smaller blocks spread them
 
 // the kAnyRun + kAnyTaps - 1 inputs of one block of taps: col[m * stride],
@@ -127,17 +127,20 @@ __global__ void __launch_bounds__(kBX * kAnyBY) fr_conv_z_kernel(const float *__
 
 // pass 2: y (axis 1), the six products.  A block takes 32 columns and kAnyRows
 // rows of a plane, puts them with their mirrored halo into shared memory, and
-// every warp computes kRun rows from there.  Reading the inputs anew for every
+// every warp computes kAnyRun rows from there.  Reading the inputs anew for every
 // run of four rows, each address mirrored again (a volume of 61 rows has hardly a
 // run with all of 49 taps inside), took 28 us at 45 x 61 x 83, radius 18 and 24;
-// this 14.  Whole filters: 120 x 120 x 100, scales 2 to 6, 514 -> 458 us; 200^3,
-// scales 4.5 and 6, 2315 -> 1990; 30 x 300 x 40, radii 18 and 40, 264 -> 204.
-constexpr int kAnyRows = 64, kAnyOut = 8;   // rows of a block and of a warp
-static_assert(kAnyRows == kAnyOut * kBY, "a run of rows per warp");
+// this 14.  One of the three inputs at a time: 80 registers and three blocks per
+// SM.  Whole filters: 120 x 120 x 100, scales 2 to 6, 514 -> 446 us; 200^3, scales
+// 4.5 and 6, 2315 -> 1839 (1991 with four z outputs per thread and all three
+// inputs at once); 30 x 300 x 40, radii 18 and 40, 264 -> 198.
+constexpr int kAnyRows = kAnyRun * kBY;   // rows of a block, a run per warp
 
-constexpr size_t fr_any_y_bytes(int r) { return sizeof(float) * 3 * (kAnyRows + 2 * r) * kBX; }
+// rows in shared memory; the last block of taps reads past the halo
+constexpr int fr_any_y_rows(int r) { return kAnyRows + 2 * r + kAnyTaps; }
+constexpr size_t fr_any_y_bytes(int r) { return sizeof(float) * 3 * fr_any_y_rows(r) * kBX; }
 
-__global__ void __launch_bounds__(kBX * kBY) fr_conv_y_kernel(const float *__restrict__ z0,
+__global__ void __launch_bounds__(kBX * kBY, 3) fr_conv_y_kernel(const float *__restrict__ z0,
                                                               const float *__restrict__ z1,
                                                               const float *__restrict__ z2, float *__restrict__ six,
                                                               int d0, int d1, int d2,
@@ -146,10 +149,10 @@ __global__ void __launch_bounds__(kBX * kBY) fr_conv_y_kernel(const float *__res
     extern __shared__ __align__(16) float any_rows[];
     const int lane = threadIdx.x, warp = threadIdx.y;
     const int x = blockIdx.x * kBX + lane, xc = min(x, d2 - 1);
-    const int y0 = blockIdx.y * kAnyRows, ya = y0 + warp * kAnyOut;
+    const int y0 = blockIdx.y * kAnyRows, ya = y0 + warp * kAnyRun;
     const int64_t s0 = (int64_t)d1 * d2, n = s0 * d0;
     const int r = tp.radius, K = 2 * r + 1;
-    const int rows = min(kAnyRows, d1 - y0) + 2 * r, part = (kAnyRows + 2 * r) * kBX;
+    const int rows = min(kAnyRows, d1 - y0) + 2 * r, part = fr_any_y_rows(r) * kBX;
     for (int z = blockIdx.z; z < d0; z += gridDim.z) {
         const int64_t plane = (int64_t)z * s0 + xc;
         for (int k = warp; k < rows; k += kBY) {
@@ -161,31 +164,34 @@ __global__ void __launch_bounds__(kBX * kBY) fr_conv_y_kernel(const float *__res
         }
         __syncthreads();
         if (ya < d1) {
-            float A[kAnyOut] = {}, B[kAnyOut] = {}, C[kAnyOut] = {}, D[kAnyOut] = {}, E[kAnyOut] = {}, F[kAnyOut] = {};
-            for (int j0 = 0; j0 < K; j0 += kAnyTaps) {
-                // rows past the last one that an output needs are read where they exist
-                const int first = warp * kAnyOut + j0, nt = K - j0;
-                float v0[kAnyOut + kAnyTaps - 1], v1[kAnyOut + kAnyTaps - 1], v2[kAnyOut + kAnyTaps - 1], t[kAnyTaps];
+            float A[kAnyRun] = {}, B[kAnyRun] = {}, C[kAnyRun] = {}, D[kAnyRun] = {}, E[kAnyRun] = {}, F[kAnyRun] = {};
+            const float *q = any_rows + warp * kAnyRun * kBX + lane;
+            for (int j0 = 0; j0 < K; j0 += kAnyTaps, q += kAnyTaps * kBX) {
+                const int nt = K - j0;
+                float v[kAnyRun + kAnyTaps - 1], t[kAnyTaps];
+                auto rows_of = [&](int k) {
 #pragma unroll
-                for (int p = 0; p < kAnyOut + kAnyTaps - 1; ++p) {
-                    const float *q = any_rows + min(first + p, rows - 1) * kBX + lane;
-                    v0[p] = q[0];
-                    v1[p] = q[part];
-                    v2[p] = q[2 * part];
-                }
+                    for (int p = 0; p < kAnyRun + kAnyTaps - 1; ++p) v[p] = q[k * part + p * kBX];
+                };
+                rows_of(0);
                 any_taps(tp, 0, j0, K, t);
-                any_fma<kAnyOut>(t, nt, v2, A);   // A = y0 Z2
-                any_fma<kAnyOut>(t, nt, v0, C);   // C = y0 Z0
-                any_fma<kAnyOut>(t, nt, v1, E);   // E = y0 Z1
+                any_fma<kAnyRun>(t, nt, v, C);   // C = y0 Z0
                 any_taps(tp, 1, j0, K, t);
-                any_fma<kAnyOut>(t, nt, v1, D);   // D = y1 Z1
-                any_fma<kAnyOut>(t, nt, v0, F);   // F = y1 Z0
+                any_fma<kAnyRun>(t, nt, v, F);   // F = y1 Z0
                 any_taps(tp, 2, j0, K, t);
-                any_fma<kAnyOut>(t, nt, v0, B);   // B = y2 Z0
+                any_fma<kAnyRun>(t, nt, v, B);   // B = y2 Z0
+                rows_of(1);
+                any_taps(tp, 0, j0, K, t);
+                any_fma<kAnyRun>(t, nt, v, E);   // E = y0 Z1
+                any_taps(tp, 1, j0, K, t);
+                any_fma<kAnyRun>(t, nt, v, D);   // D = y1 Z1
+                rows_of(2);
+                any_taps(tp, 0, j0, K, t);
+                any_fma<kAnyRun>(t, nt, v, A);   // A = y0 Z2
             }
             if (x < d2) {
 #pragma unroll
-                for (int o = 0; o < kAnyOut; ++o) {
+                for (int o = 0; o < kAnyRun; ++o) {
                     if (ya + o < d1) {
                         const int64_t i = plane + (int64_t)(ya + o) * d2;
                         six[i] = A[o];
