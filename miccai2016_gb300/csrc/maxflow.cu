@@ -314,6 +314,17 @@ struct EventPool {
             if (e) cudaEventDestroy(e);
     }
 };
+
+// Iterations between two looks at the stopping state: whole check intervals, at
+// least `least` iterations, a multiple of `unit`, no more than the solve has.
+// 64-bit until it is cut: an update of 2^31 - 1 ("check once") is in order.
+inline int mf_chunk(int num_iter, int update, int least, int unit)
+{
+    int64_t c = std::max<int64_t>((int64_t)update * std::max(1, 64 / update), least);
+    c = (c + unit - 1) / unit * unit;
+    return (int)std::min<int64_t>(c, std::max(num_iter, 1));
+}
+inline int mf_chunk_end(int it, int chunk, int num_iter) { return (int)std::min<int64_t>(num_iter, (int64_t)it + chunk); }
 }  // namespace
 
 namespace {
@@ -383,16 +394,14 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
     int launches = 3;
 
     const int num_iter = params->num_iter, update = params->update;
-    // iterations between two looks at the stopping state: even, so that pairs
-    // start at even iterations; without a bound only a NaN residual stops
-    int chunk = update * std::max(1, 64 / update);
-    chunk += chunk & 1;
-    if (!(params->error_bound > 0.0)) chunk = std::max(chunk, 1024);
+    // even, so that pairs start at even iterations; without a bound only a NaN
+    // residual stops
+    const int chunk = mf_chunk(num_iter, update, params->error_bound > 0.0 ? 1 : 1024, 2);
     const bool timing = stats && stats->time_kernels;
     const bool pdl = !(stats && (stats->flags & M16_SOLVE_NO_PDL));
     std::unique_ptr<EventPool> pool;
     if (timing) {
-        pool.reset(new EventPool(std::min(num_iter, chunk) + 2));
+        pool.reset(new EventPool(chunk + 2));
         if (!pool->ok) return M16_ERR_CUDA;
     }
     int it = 0;
@@ -408,7 +417,7 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
     MfCtrl hctrl;
     hctrl.stopped = 0;
     while (it < num_iter) {
-        const int end = std::min(num_iter, it + chunk), begin = it;
+        const int end = mf_chunk_end(it, chunk, num_iter), begin = it;
         int slots = 0;
         while (it < end) {
             const int count = std::min(2, num_iter - it);
@@ -546,7 +555,7 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
     const bool sup = labels != nullptr;
     const double inv_norm = 1.0 / ((double)n * rcc);
     const int update = params->update;
-    const int chunk = update * std::max(1, 64 / update);
+    const int chunk = mf_chunk(params->num_iter, update, 1, 1);
 
     const bool timing = stats && stats->time_kernels;
     const bool pdl = !(stats && (stats->flags & M16_SOLVE_NO_PDL));
@@ -562,7 +571,7 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
     hctrl.stopped = 0;
     int it = 0;
     while (it < params->num_iter) {
-        const int end = std::min(params->num_iter, it + chunk);
+        const int end = mf_chunk_end(it, chunk, params->num_iter);
         // per launch slot: its iteration, for the timing
         std::vector<int> slot_it;
         while (it < end) {
