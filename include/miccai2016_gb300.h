@@ -31,7 +31,7 @@ extern "C" {
 #define M16_ERR_BAD_ARG 2       /* a NULL pointer, a non-finite or out-of-range parameter */
 #define M16_ERR_WORKSPACE 3     /* workspace NULL, misaligned or smaller than required */
 #define M16_ERR_CUDA 4          /* a CUDA runtime call failed */
-#define M16_ERR_TIMEOUT 5       /* a bounded device-side wait gave up */
+#define M16_ERR_TIMEOUT 5       /* a bounded device-side wait gave up (a bulk copy of the tile sweeps: after 0.4 to 1 s); outputs are not valid */
 #define M16_ERR_TOO_LARGE 6     /* the request exceeds a fixed capacity: the scratch of m16_maxflow_solve_static
                                    or the work table of a server (max_work_items) */
 
@@ -305,7 +305,9 @@ int m16_server_create(const m16_cut_params *params, int32_t max_slots, int32_t m
 int m16_server_admit(m16_server *s, const m16_serve_request *req, int32_t *admitted);
 
 /* The iterations up to the next check of every resident request (update of
- * them; after its last check those that remain), then retirement. */
+ * them; after its last check those that remain), then retirement.  After
+ * M16_ERR_TIMEOUT the server takes no more: admit and step return it, and poll
+ * does once the finished requests have been handed out. */
 int m16_server_step(m16_server *s);
 
 /* Requests whose u has reached the host since the last call: tags,

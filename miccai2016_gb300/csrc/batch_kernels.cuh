@@ -55,7 +55,7 @@ namespace {
 constexpr int kBX = 32, kBY = 8, kTile = kBX * kBY;
 constexpr int kSetupBlocks = 4 * kSMs;
 
-constexpr unsigned kStopped = 1u, kBuffer = 2u;   // bits of an instance's state word
+constexpr unsigned kStopped = 1u, kBuffer = 2u;   // bits of an instance's state word (kStopped: also tile_fail's)
 
 struct InstCtrl {
     int stopped;
@@ -78,7 +78,8 @@ struct InstDev {
 
 // an instance of the tile sweeps
 struct TileDev {
-    TileView V;              // all but the buffers
+    TileView V;              // all but the buffers and fail
+    TileFail fail;
     const CUtensorMap *mh[2], *mu[2];
     float4 *h[2];
     float2 *u[2];
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) bt_tile_kern
     V.mu = T.mu[b];
     V.ho = T.h[1 - b];
     V.uo = T.u[1 - b];
+    V.fail = &T.fail;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         tile_acquire(V.mh);
         tile_acquire(V.mu);

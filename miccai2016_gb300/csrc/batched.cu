@@ -293,7 +293,7 @@ int batch_prepare(BatchRun &B, const m16_batch_volume *vols, int nvol, const m16
         t.V.w = w;
         t.V.nid2 = nid2;
         t.V.labels = nullptr;
-        t.V.err = (int *)field(L.err);
+        t.fail = TileFail{(int *)field(L.err), (int *)field(L.state) + i};
         CUtensorMap *m = B.hmaps.data() + 6 * nvol + 5 * i;
         CUtensorMap *dm = dmaps + 6 * nvol + 5 * i, *dv = dmaps + 6 * v;
         bool ok = true;

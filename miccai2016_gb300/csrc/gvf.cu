@@ -482,7 +482,7 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
     a.ndt = -(float)dt;
     a.comp = tile_voxels(d0, d1, d2);
     a.partials = (float *)(ws + L.partials);
-    a.err = &ctrl->error;
+    a.fail = TileFail{&ctrl->error, &ctrl->stopped};
     CUtensorMap mg[2];
     bool ok = gvf_map(&a.mv, ws + L.v, d0, d1, a.pitch, kGvfVW, tile_rows);
     for (int b = 0; b < 2; ++b) ok = ok && gvf_map(&mg[b], g[b], d0, d1, a.pitch, kGvfGW, tile_rows + 2);

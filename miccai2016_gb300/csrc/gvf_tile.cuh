@@ -58,7 +58,7 @@ struct GvfTileArgs {
     float *partials;                // per iteration: per block
     int checks;                     // bit k: |delta| of iteration k is summed
     const GvfCtrl *ctrl;            // null: run whatever the state
-    int *err;
+    TileFail fail;
 };
 
 template <int K, bool RESP>
@@ -174,7 +174,10 @@ __global__ void __launch_bounds__(kTileLanes *GvfShape<RESP>::NW, GvfShape<RESP>
             __syncthreads();   // the last step's edges are stored, its slots read
             const unsigned f = (unsigned)(z - (zs - 1));
             // the slot last read a step ago: v of the last stage, g of the first
-            if (copier && z - Lag >= zs - 1 && z - Lag + S <= zl) fill(z - Lag + S);
+            if (copier && z - Lag >= zs - 1 && z - Lag + S <= zl) {
+                if (ok) fill(z - Lag + S);
+                else bar_release(&M.full[(f - Lag) % S], ((f - Lag + S) / S) & 1u);
+            }
             if (z <= zl) {
                 wait(z);
                 const auto &cur = M.slot[f % S];
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(kTileLanes *GvfShape<RESP>::NW, GvfShape<RESP>
             }
         }
     }
-    if (!ok) *a.err = 1;
+    if (!ok) tile_fail(a.fail);
     if (CHECK) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {

@@ -354,7 +354,6 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
     V.rcc = (float)rcc;
     V.ircc = (float)(1.0 / rcc);
     V.labels = labels;
-    V.err = &ctrl->error;
     // the two directions of a sweep: buffer k read, the other written
     MfTileArgs args[2];
     for (int k = 0; k < 2; ++k) {
@@ -365,6 +364,7 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
         a.nx = L.nx; a.ny = L.ny; a.zc = L.zc;
         a.partials = (float *)(ws + L.partials);
         a.stopped = &ctrl->stopped;
+        a.fail = TileFail{&ctrl->error, &ctrl->stopped};
         bool ok = tile_map(&a.mh, ws + L.h[k], d0, d1, V.pitch, 4, kTileRows + 1) &&
                   tile_map(&a.mu, ws + L.u[k], d0, d1, V.pitch, 2, kTileRows) &&
                   tile_map(&a.mcaps, ws + L.caps, d0, d1, V.pitch, 2, kTileRows);

@@ -19,6 +19,7 @@ struct MfTileArgs {
     int nx, ny, zc;
     float *partials;        // per block: iteration 0, then iteration 1
     const int *stopped;     // null: run whatever the solve's state
+    TileFail fail;
 };
 
 template <int K, int METRIC, int ASRC, bool SUP, bool CHECK>
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(kTileLanes *kTileNW, kTileBlocks) mf_tile_kern
     tile_init(M);
     TileView V = a.V;
     V.mh = &a.mh; V.mu = &a.mu; V.mdir = &a.mdir; V.meig = &a.meig; V.mcaps = &a.mcaps; V.mrad = &a.mrad;
+    V.fail = &a.fail;
     const int bx = blockIdx.x % a.nx, t = blockIdx.x / a.nx;
     const int by = t % a.ny, za = t / a.ny * a.zc;
     float acc[2] = {0.f, 0.f};

@@ -247,6 +247,7 @@ struct m16_server {
     int64_t processed = 0;           // steps whose stop masks have been read (all steps < processed)
     int64_t voxel_iterations = 0;    // iterations that ran, times each request's voxels
     double gpu_ms = 0.0;             // device time of the steps' kernels
+    bool failed = false;             // a step's copies did not arrive: no further admission or step
     struct Done {
         int64_t tag;
         int iterations;
@@ -370,7 +371,7 @@ int process_step(m16_server *s, int64_t idx);
 // last requests come back without another step call.
 void collect(m16_server *s)
 {
-    while (s->processed < s->steps && cudaEventQuery(s->ctrl_ev[s->processed & 1]) == cudaSuccess)
+    while (!s->failed && s->processed < s->steps && cudaEventQuery(s->ctrl_ev[s->processed & 1]) == cudaSuccess)
         if (process_step(s, s->processed) != M16_OK) break;
     for (int k = 0; k < s->max_slots; ++k) {
         Slot &sl = s->slots[k];
@@ -448,6 +449,7 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
 {
     if (!s || !req || !admitted) return M16_ERR_BAD_ARG;
     *admitted = 0;
+    if (s->failed) return M16_ERR_TIMEOUT;
     if (req->d0 < 1 || req->d1 < 1 || req->d2 < 1) return M16_ERR_BAD_SHAPE;
     if ((int64_t)req->d0 * req->d1 * req->d2 > (int64_t)INT32_MAX) return M16_ERR_BAD_SHAPE;
     if (!req->img || !req->quat3 || !req->cs || !req->ct || !req->u) return M16_ERR_BAD_ARG;
@@ -455,6 +457,7 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
     for (int k = 0; k < 3; ++k)
         if (!(req->scaling[k] > 0.0) || !(req->sqevals[k] > 0.0)) return M16_ERR_BAD_ARG;
     collect(s);
+    if (s->failed) return M16_ERR_TIMEOUT;
     if (s->free_slots.empty()) return M16_OK;
     TileView view = TileView();
     int axis;
@@ -536,7 +539,7 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
         t.V.w = w;
         t.V.nid2 = nid2;
         t.V.labels = nullptr;
-        t.V.err = (int *)(s->ws + s->T.err);
+        t.fail = TileFail{(int *)(s->ws + s->T.err), (int *)(s->ws + s->T.state) + k};
         CUtensorMap *dm = (CUtensorMap *)(s->ws + s->T.maps) + 8 * k;
         bool ok = true;
         for (int b = 0; b < 2; ++b) {
@@ -644,7 +647,8 @@ int process_step(m16_server *s, int64_t idx)
     float step_ms = 0.f;
     M16_CUDA_TRY(cudaEventElapsedTime(&step_ms, s->t_start[b], s->t_end[b]));
     s->gpu_ms += step_ms;
-    if (s->err_h[b]) return M16_ERR_TIMEOUT;
+    if (s->err_h[b]) s->failed = true;
+    if (s->failed) return M16_ERR_TIMEOUT;
     for (const auto &entry : s->step_list[b]) {
         const int k = entry.first, target = entry.second;
         Slot &sl = s->slots[k];
@@ -671,7 +675,9 @@ int process_step(m16_server *s, int64_t idx)
 extern "C" int m16_server_step(m16_server *s)
 {
     if (!s) return M16_ERR_BAD_ARG;
+    if (s->failed) return M16_ERR_TIMEOUT;
     collect(s);
+    if (s->failed) return M16_ERR_TIMEOUT;
     if (s->dirty) {
         const int r = rebuild(s);
         if (r != M16_OK) return r;
@@ -736,7 +742,7 @@ extern "C" int m16_server_poll(m16_server *s, int64_t *tags, int32_t *iterations
     }
     s->done.erase(s->done.begin(), s->done.begin() + cnt);
     *n = cnt;
-    return M16_OK;
+    return s->failed && cnt == 0 ? M16_ERR_TIMEOUT : M16_OK;
 }
 
 extern "C" int m16_server_get_info(const m16_server *s, m16_server_info *info)
