@@ -537,13 +537,14 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
     if (h.error) return M16_ERR_TIMEOUT;
     const int done = h.stopped ? h.iterations : first_iter + n_iters;   // total iterations so far
     int buf = buf0;
+    bool again = false;
     if (!was_stopped) {
         const int ran = done - first_iter;
         buf = (buf0 + (int)div_up(ran, pass)) & 1;
         // stopped inside a sweep: its iterations up to there again, from the
         // buffer it read
-        if (h.stopped && ran % pass && ran < n_iters)
-            M16_CUDA_TRY(sweep(done - ran % pass, ran % pass, 1 - buf, true));
+        again = h.stopped && ran % pass && ran < n_iters;
+        if (again) M16_CUDA_TRY(sweep(done - ran % pass, ran % pass, 1 - buf, true));
     }
     gvf_tile_output_kernel<<<blocks1d, 256, 0, st>>>(g[buf], d2, rows, normalize, buf, ctrl, g3);
     M16_CUDA_TRY(cudaGetLastError());
@@ -554,8 +555,10 @@ int gvf_run_tiles(const float *v3, const float *response, int d0, int d1, int d2
         const int cnt = std::min(std::min(h.n_checks, mags_cap), L.cap);
         if (cnt > 0) M16_CUDA_TRY(cudaMemcpyAsync(mags, mlog, (size_t)cnt * 8, cudaMemcpyDeviceToHost, st));
     }
+    int late = 0;   // a copy of the iterations that ran again
+    if (again) M16_CUDA_TRY(cudaMemcpyAsync(&late, &ctrl->error, sizeof(int), cudaMemcpyDeviceToHost, st));
     M16_CUDA_TRY(cudaStreamSynchronize(st));
-    return M16_OK;
+    return late ? M16_ERR_TIMEOUT : M16_OK;
 }
 
 }  // namespace

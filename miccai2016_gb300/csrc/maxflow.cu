@@ -456,7 +456,8 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
     const int ran = hctrl.stopped ? hctrl.iterations : it;
     // stopped by the check of a pair's first iteration: that one again, alone,
     // from the buffer the pair read
-    if (ran & 1 && ran < num_iter) {
+    const bool again = ran & 1 && ran < num_iter;
+    if (again) {
         M16_CUDA_TRY(sweep(1, false, (ran >> 1) & 1, true));
         ++launches;
     }
@@ -477,8 +478,10 @@ int maxflow_solve_tiles(const float *img, const float *quat3, const double *sqev
         const int cnt = std::min(std::min(hctrl.n_checks, residuals_cap), L.resid_cap);
         if (cnt > 0) M16_CUDA_TRY(cudaMemcpyAsync(residuals, resid, (size_t)cnt * 8, cudaMemcpyDeviceToHost, st));
     }
+    int late = 0;   // a copy of the iteration that ran again
+    if (again) M16_CUDA_TRY(cudaMemcpyAsync(&late, &ctrl->error, sizeof(int), cudaMemcpyDeviceToHost, st));
     M16_CUDA_TRY(cudaStreamSynchronize(st));
-    return M16_OK;
+    return late ? M16_ERR_TIMEOUT : M16_OK;
 }
 
 }  // namespace
