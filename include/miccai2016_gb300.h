@@ -203,8 +203,17 @@ typedef struct m16_batch_instance {
     float *u;             /* N output */
 } m16_batch_instance;
 
-/* Workspace bytes of m16_batch_solve (0 when the descriptors are invalid). */
+/* Workspace bytes of m16_batch_solve and m16_batch_begin (0 when the descriptors
+ * are invalid).  m16_batch_solve runs in less, down to
+ * m16_batch_workspace_bytes_min: it takes the instances in cohorts that fit, and
+ * one that does not fit alone with a single state buffer and slower sweeps.
+ * m16_batch_begin_min runs in less, down to m16_batch_steps_bytes_min, with a
+ * single state buffer for every instance. */
 size_t m16_batch_workspace_bytes(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
+                                 int32_t ninst);
+size_t m16_batch_workspace_bytes_min(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
+                                     int32_t ninst);
+size_t m16_batch_steps_bytes_min(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
                                  int32_t ninst);
 
 /*
@@ -243,6 +252,9 @@ typedef struct m16_batch m16_batch;
 int m16_batch_begin(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst, int32_t ninst,
                     const m16_cut_params *params, void *workspace, size_t workspace_bytes, void *stream,
                     m16_batch **out);
+int m16_batch_begin_min(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst, int32_t ninst,
+                        const m16_cut_params *params, void *workspace, size_t workspace_bytes, void *stream,
+                        m16_batch **out);
 int m16_batch_iterate(m16_batch *b, int32_t count, void *stream);
 int m16_batch_end(m16_batch *b, int32_t *iterations, double *residuals, void *stream);
 

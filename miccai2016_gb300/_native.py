@@ -177,12 +177,17 @@ def _declare(L):
     L.m16_adjust_nonridge_signs_indexed.argtypes = [_vp, _i32, _i32, _i32, _vp, _vp, _i64, _vp, _vp, _sz, _vp]
     L.m16_batch_workspace_bytes.restype = _sz
     L.m16_batch_workspace_bytes.argtypes = [ctypes.POINTER(BatchVolume), _i32, ctypes.POINTER(BatchInstance), _i32]
+    for least in (L.m16_batch_workspace_bytes_min, L.m16_batch_steps_bytes_min):
+        least.restype = _sz
+        least.argtypes = L.m16_batch_workspace_bytes.argtypes
     L.m16_batch_solve.restype = ctypes.c_int
     L.m16_batch_solve.argtypes = [ctypes.POINTER(BatchVolume), _i32, ctypes.POINTER(BatchInstance), _i32,
                                   ctypes.POINTER(CutParams), _vp, _vp, _vp, _sz, _vp, ctypes.POINTER(SolveStats)]
     L.m16_batch_begin.restype = ctypes.c_int
     L.m16_batch_begin.argtypes = [ctypes.POINTER(BatchVolume), _i32, ctypes.POINTER(BatchInstance), _i32,
                                   ctypes.POINTER(CutParams), _vp, _sz, _vp, ctypes.POINTER(_vp)]
+    L.m16_batch_begin_min.restype = ctypes.c_int
+    L.m16_batch_begin_min.argtypes = L.m16_batch_begin.argtypes
     L.m16_batch_iterate.restype = ctypes.c_int
     L.m16_batch_iterate.argtypes = [_vp, _i32, _vp]
     L.m16_batch_end.restype = ctypes.c_int

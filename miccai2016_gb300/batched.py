@@ -20,6 +20,19 @@ from . import _native as N
 from .continuous_cut_anisotropic_gpu import CmfCutQAnisotropicGpu
 
 
+def _workspace(nbytes, least, between=True):
+    """nbytes of workspace or, where the device has no room for them, half as
+    many and so on (between), at last the least that the call accepts."""
+    torch = N.torch_mod()
+    while True:
+        try:
+            return N.workspace(nbytes)
+        except torch.cuda.OutOfMemoryError:
+            if nbytes <= least:
+                raise
+            nbytes = max(least, nbytes // 2) if between else least
+
+
 class BatchedCut(object):
     """Batch solver with the cut parameters of CmfCutQAnisotropicGpu.CutParameters."""
 
@@ -83,7 +96,7 @@ class BatchedCut(object):
             raise ValueError("invalid batch description")
         if self._ws is None or self._ws.numel() < nbytes:
             self._ws = None
-            self._ws = N.workspace(nbytes)
+            self._ws = _workspace(nbytes, L.m16_batch_workspace_bytes_min(vd, nv, idesc, ni))
         iters = (ctypes.c_int32 * ni)()
         res = (ctypes.c_double * ni)()
         stats = N.SolveStats(int(bool(time_kernels)), 0, 0, 0, 0.0, 0.0,
@@ -148,7 +161,8 @@ class BatchSteps(object):
         nbytes = L.m16_batch_workspace_bytes(self._vd, len(volumes), self._idesc, len(instances))
         if nbytes == 0:
             raise ValueError("invalid batch description")
-        self._ws = N.workspace(nbytes)
+        self._ws = _workspace(nbytes, L.m16_batch_steps_bytes_min(self._vd, len(volumes), self._idesc, len(instances)),
+                              between=False)
         self._n = len(instances)
         # every (non-capturing) stream the batch's work went to: end() orders
         # itself after all of them, whichever stream is current then
@@ -156,9 +170,9 @@ class BatchSteps(object):
         self._last_stream = None
         self._note_stream()
         h = ctypes.c_void_p()
-        N.check("m16_batch_begin", L.m16_batch_begin(self._vd, len(volumes), self._idesc, self._n,
-                                                     ctypes.byref(self._cp), N.ptr(self._ws), self._ws.numel(),
-                                                     N.stream_ptr(), ctypes.byref(h)))
+        begin = L.m16_batch_begin if self._ws.numel() >= nbytes else L.m16_batch_begin_min
+        N.check("m16_batch_begin", begin(self._vd, len(volumes), self._idesc, self._n, ctypes.byref(self._cp),
+                                         N.ptr(self._ws), self._ws.numel(), N.stream_ptr(), ctypes.byref(h)))
         self._h = h
         self.iterations = None
         self.residuals = None

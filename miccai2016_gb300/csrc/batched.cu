@@ -18,13 +18,12 @@ namespace {
 
 // ---- host side --------------------------------------------------------------
 
-// Double-buffered state up to this many bytes; a batch that would take more is
-// solved in cohorts that fit, one after the other (the step interface, which
-// holds every instance at once, takes the compact sweeps instead).
-#ifndef M16_BATCH_PAIR_BUDGET
-#define M16_BATCH_PAIR_BUDGET ((size_t)128 << 30)
-#endif
-constexpr size_t kPairBudget = M16_BATCH_PAIR_BUDGET;
+// Double-buffered state is asked for up to this many bytes.  In a workspace that
+// does not hold the whole batch that way it is solved in cohorts that fit, one
+// after the other, an instance that does not even fit alone by the compact
+// sweeps; the step interface, which holds every instance at once, takes the
+// compact sweeps for all of them.
+constexpr size_t kPairBudget = (size_t)128 << 30;
 
 // Tile shapes of the autotuner, named by their target blocks per SM: 16 is the
 // chunk of z of batch_chunk's rule, 8 twice and 32 half of it.  The candidates
@@ -192,6 +191,14 @@ inline size_t batch_bytes(const m16_batch_volume *vols, int nvol, const m16_batc
     const size_t full = batch_layout(vols, nvol, inst, 0, ninst, false).total;
     if (full <= kPairBudget) return full;
     return std::max(kPairBudget, batch_layout(vols, nvol, inst, 0, ninst, true).total);
+}
+
+// The least that m16_batch_solve runs in: every instance alone, compact
+inline size_t batch_bytes_min(const m16_batch_volume *vols, int nvol, const m16_batch_instance *inst, int ninst)
+{
+    size_t least = 0;
+    for (int i = 0; i < ninst; ++i) least = std::max(least, batch_layout(vols, nvol, inst, i, i + 1, true).total);
+    return least;
 }
 
 // A batch's descriptors on host and device and its work list
@@ -695,6 +702,20 @@ extern "C" size_t m16_batch_workspace_bytes(const m16_batch_volume *vols, int32_
     return batch_bytes(vols, nvol, inst, ninst);
 }
 
+extern "C" size_t m16_batch_workspace_bytes_min(const m16_batch_volume *vols, int32_t nvol,
+                                                const m16_batch_instance *inst, int32_t ninst)
+{
+    if (!batch_args_ok(vols, nvol, inst, ninst)) return 0;
+    return batch_bytes_min(vols, nvol, inst, ninst);
+}
+
+extern "C" size_t m16_batch_steps_bytes_min(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
+                                            int32_t ninst)
+{
+    if (!batch_args_ok(vols, nvol, inst, ninst)) return 0;
+    return batch_layout(vols, nvol, inst, 0, ninst, true).total;
+}
+
 extern "C" int m16_batch_solve(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
                                int32_t ninst, const m16_cut_params *params, int32_t *iterations, double *residuals,
                                void *workspace, size_t workspace_bytes, void *stream, m16_solve_stats *stats)
@@ -707,7 +728,7 @@ extern "C" int m16_batch_solve(const m16_batch_volume *vols, int32_t nvol, const
         for (int c : kTuneBps) known = known || c == stats->blocks_per_sm;
         if (!known) return M16_ERR_BAD_ARG;
     }
-    if (!workspace || workspace_bytes < batch_bytes(vols, nvol, inst, ninst) || ((uintptr_t)workspace & 255))
+    if (!workspace || workspace_bytes < batch_bytes_min(vols, nvol, inst, ninst) || ((uintptr_t)workspace & 255))
         return M16_ERR_WORKSPACE;
     if (stats) {
         stats->launches = stats->p_launches = stats->u_launches = stats->pair_launches = 0;
@@ -751,20 +772,23 @@ struct m16_batch {
     int iterations_run = 0;          // iterations enqueued by m16_batch_iterate
 };
 
-extern "C" int m16_batch_begin(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
-                               int32_t ninst, const m16_cut_params *params, void *workspace, size_t workspace_bytes,
-                               void *stream, m16_batch **out)
+// least: the workspace may be too small for the size that m16_batch_workspace_bytes gives
+static int batch_begin(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst, int32_t ninst,
+                       const m16_cut_params *params, void *workspace, size_t workspace_bytes, void *stream, bool least,
+                       m16_batch **out)
 {
     if (!out) return M16_ERR_BAD_ARG;
     *out = nullptr;
     if (!params || params->update < 1 || params->num_iter < 0 || !(params->cc > 0.0)) return M16_ERR_BAD_ARG;
     if (!batch_args_ok(vols, nvol, inst, ninst)) return M16_ERR_BAD_ARG;
-    if (!workspace || workspace_bytes < batch_bytes(vols, nvol, inst, ninst) || ((uintptr_t)workspace & 255))
-        return M16_ERR_WORKSPACE;
+    if (!workspace || ((uintptr_t)workspace & 255)) return M16_ERR_WORKSPACE;
+    if (!least && workspace_bytes < batch_bytes(vols, nvol, inst, ninst)) return M16_ERR_WORKSPACE;
+    BatchLayout layout = batch_layout(vols, nvol, inst, 0, ninst, false);
+    if (layout.total > workspace_bytes) layout = batch_layout(vols, nvol, inst, 0, ninst, true);
+    if (layout.total > workspace_bytes) return M16_ERR_WORKSPACE;
     m16_batch *b = new m16_batch();
     BatchRun &B = b->B;
-    B.L = batch_layout(vols, nvol, inst, 0, ninst, false);
-    if (B.L.total > workspace_bytes) B.L = batch_layout(vols, nvol, inst, 0, ninst, true);
+    B.L = layout;
     b->params = *params;
     cudaStream_t st = (cudaStream_t)stream;
     int launches = 0;
@@ -779,6 +803,20 @@ extern "C" int m16_batch_begin(const m16_batch_volume *vols, int32_t nvol, const
     }
     *out = b;
     return M16_OK;
+}
+
+extern "C" int m16_batch_begin(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
+                               int32_t ninst, const m16_cut_params *params, void *workspace, size_t workspace_bytes,
+                               void *stream, m16_batch **out)
+{
+    return batch_begin(vols, nvol, inst, ninst, params, workspace, workspace_bytes, stream, false, out);
+}
+
+extern "C" int m16_batch_begin_min(const m16_batch_volume *vols, int32_t nvol, const m16_batch_instance *inst,
+                                   int32_t ninst, const m16_cut_params *params, void *workspace, size_t workspace_bytes,
+                                   void *stream, m16_batch **out)
+{
+    return batch_begin(vols, nvol, inst, ninst, params, workspace, workspace_bytes, stream, true, out);
 }
 
 extern "C" int m16_batch_iterate(m16_batch *b, int32_t count, void *stream)
