@@ -103,7 +103,8 @@ inline BatchLayout batch_layout(const m16_batch_volume *vols, int nvol, const m1
         int axis;
         const int metric = tile_metric(I.sqevals, view, &axis);
         L.axis.push_back(axis);
-        if (compact || !tile_shape_ok(V.d0, V.d1, V.d2)) {
+        if (compact || !tile_shape_ok(V.d0, V.d1, V.d2) ||
+            !tile_rows_ok(metric, V.d0, V.d1, V.d2, kSmallInstance)) {
             P.compact = true;
             L.kind.push_back(I.alpha ? kCompactAlpha : kCompactExp);
             continue;

@@ -514,7 +514,11 @@ static int maxflow_solve_impl(const float *img, const float *quat3, const double
     // Two iterations a pass over 72 bytes a voxel (256^3: 95 us an iteration)
     // against two passes an iteration over 88 (228 us); the two sweeps take half
     // the workspace and any volume size.
-    if (tile_shape_ok(d0, d1, d2) && !(stats && stats->path == M16_PATH_TWO_SWEEPS)) {
+    TileView view = TileView();
+    int axis;
+    const int metric = sqevals3 ? tile_metric(sqevals3, view, &axis) : kMetricField;
+    if (tile_shape_ok(d0, d1, d2) && tile_rows_ok(metric, d0, d1, d2, kSmallSolve) &&
+        !(stats && stats->path == M16_PATH_TWO_SWEEPS)) {
         const MfTileLayout T = mf_tile_layout(d0, d1, d2, params->num_iter, params->update, sqevals3 == nullptr);
         if (workspace_bytes >= T.total)
             return maxflow_solve_tiles(img, quat3, sqevals3, sqeigs, alpha, alpha_scalar, cs, ct, labels, d0, d1, d2,

@@ -390,7 +390,11 @@ extern "C" size_t m16_server_request_bytes(int32_t d0, int32_t d1, int32_t d2, i
 {
     (void)has_alpha;   // the alpha field takes the place of |grad I|^2
     if (d0 < 1 || d1 < 1 || d2 < 1 || (int64_t)d0 * d1 * d2 > (int64_t)INT32_MAX) return 0;
-    return req_layout(d0, d1, d2, !tile_shape_ok(d0, d1, d2), false).total;
+    const bool tiled = tile_shape_ok(d0, d1, d2);
+    const size_t bytes = req_layout(d0, d1, d2, !tiled, false).total;
+    // with few rows the sweeps depend on the eigenvalues
+    if (!tiled || tile_rows_ok(kMetricConst, d0, d1, d2, kSmallInstance)) return bytes;
+    return std::max(bytes, req_layout(d0, d1, d2, true, false).total);
 }
 
 extern "C" size_t m16_server_table_bytes(int32_t max_slots, int32_t max_work_items)
@@ -464,7 +468,9 @@ extern "C" int m16_server_admit(m16_server *s, const m16_serve_request *req, int
     const int metric = tile_metric(req->sqevals, view, &axis);
     tile_view(view, req->d0, req->d1, req->d2, req->scaling, s->params);
     const bool rad = metric == kMetricConst;   // a radius field beside the quaternions
-    ReqLayout R = req_layout(req->d0, req->d1, req->d2, !tile_shape_ok(req->d0, req->d1, req->d2), rad);
+    const bool tiled = tile_shape_ok(req->d0, req->d1, req->d2) &&
+                       tile_rows_ok(metric, req->d0, req->d1, req->d2, kSmallInstance);
+    ReqLayout R = req_layout(req->d0, req->d1, req->d2, !tiled, rad);
     size_t block;
     if (R.tiles > s->max_work || !s->arena.alloc(R.total, &block)) {
         // A request that the tile sweeps' fields do not fit even alone takes the
