@@ -377,6 +377,7 @@ inline int gvf_warps(bool resp) { return resp ? GvfShape<true>::NW : GvfShape<fa
 // blocks of a launch of k iterations
 struct GvfTileGrid {
     int nx, ny, zc, blocks;
+    int64_t steps;   // waves x marched planes
 };
 
 inline GvfTileGrid gvf_tile_grid(int d0, int d1, int d2, int k, bool resp)
@@ -400,10 +401,29 @@ inline GvfTileGrid gvf_tile_grid(int d0, int d1, int d2, int k, bool resp)
         if (zc == 1) break;
     }
     G.blocks = (int)(tiles * div_up(d0, G.zc));
+    G.steps = cost;
     return G;
 }
 
-inline bool gvf_tile_ok(int d0, int d1, int d2) { return d2 >= 2 && tile_shape_ok(d0, d1, d2); }
+// Whether the tile sweeps run.  They need two columns, and are the slower ones
+// where the plain sweep keeps to the 3 us of a launch (up to a block or two per
+// SM) and a pass of tiles does not make up for its march: 60 iterations, plain and
+// tiles, with a response 48 x 24 x 24 197 and 220 us, 64 x 16 x 64 (two planes a block)
+// 222 and 243, 24 x 24 x 100 (two blocks per SM) 224 and 223, 2 x 128 x 128 209 and 174;
+// without one 64 x 8 x 64 (tiles on both halves of an SM) 203 and 247, 24^3 193 and
+// 194.  And where few rows fill little of a block and the launch is not a short
+// one: with a response 512 x 8 x 512 1093 and 1938, 512 x 12 x 512 1953 and 1971, 256 x 8 x
+// 256 569 and 633; without 512 x 8 x 512 1020 and 1429, 512 x 10 x 512 1555 and 1540, 256 x
+// 8 x 256 567 and 516.
+inline bool gvf_tile_ok(int d0, int d1, int d2, bool resp)
+{
+    if (d2 < 2 || !tile_shape_ok(d0, d1, d2)) return false;
+    const GvfTileGrid G = gvf_tile_grid(d0, d1, d2, gvf_iterations(resp), resp);
+    const int64_t plain = div_up(d2, kBX) * div_up(d1, kBY) * d0;   // blocks of one plane each
+    if (resp ? d1 < 12 && G.steps > 9 : d1 < 10 && G.steps > 13) return false;
+    if (resp) return d0 <= 2 || plain > (G.zc > 1 ? 2 : 1) * kSMs;
+    return G.blocks <= kSMs || plain > 2 * kSMs;
+}
 
 inline GvfTileLayout gvf_tile_layout(int d0, int d1, int d2, int has_response, int mags_cap)
 {
@@ -570,8 +590,11 @@ extern "C" size_t m16_gvf_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, in
                                           int32_t mags_cap)
 {
     if (d0 < 1 || d1 < 1 || d2 < 1) return 0;
-    if (gvf_tile_ok(d0, d1, d2)) return gvf_tile_layout(d0, d1, d2, has_response, mags_cap).total;
-    return gvf_layout(d0, d1, d2, has_response, mags_cap).total;
+    size_t bytes = 0;   // one that holds a response does without one too
+    for (int r = 0; r <= (has_response ? 1 : 0); ++r)
+        bytes = std::max(bytes, gvf_tile_ok(d0, d1, d2, r != 0) ? gvf_tile_layout(d0, d1, d2, r, mags_cap).total
+                                                                : gvf_layout(d0, d1, d2, r, mags_cap).total);
+    return bytes;
 }
 
 extern "C" int m16_gvf_run(const float *v3, const float *response, int32_t d0, int32_t d1, int32_t d2,
@@ -586,7 +609,7 @@ extern "C" int m16_gvf_run(const float *v3, const float *response, int32_t d0, i
     if (update < 1 || first_iter < 0 || n_iters < 0 || !(dt > 0.0) || !(mu >= 0.0)) return M16_ERR_BAD_ARG;
     for (int k = 0; k < 3; ++k)
         if (!(voxel_size[k] > 0.0)) return M16_ERR_BAD_ARG;
-    if (gvf_tile_ok(d0, d1, d2)) {
+    if (gvf_tile_ok(d0, d1, d2, response != nullptr)) {
         const GvfTileLayout T = gvf_tile_layout(d0, d1, d2, response != nullptr, mags_cap);
         if (!workspace || workspace_bytes < T.total || ((uintptr_t)workspace & 255)) return M16_ERR_WORKSPACE;
         return gvf_run_tiles(v3, response, d0, d1, d2, voxel_size, mu, dt, first_iter, n_iters, update, tol, normalize,
