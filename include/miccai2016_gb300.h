@@ -116,7 +116,8 @@ typedef struct m16_solve_stats {
     int32_t blocks_per_sm; /* out (m16_batch_solve): the sweeps' tile shape in use at the end: 16 is the
                               default chunk of planes per block, 8 twice and 32 half of it; in, with
                               M16_BATCH_NO_TUNE: 8, 16 or 32 fixes that shape (0: the default) */
-    int32_t pair_launches; /* out: launches of two iterations that ran (m16_batch_solve: time_kernels only) */
+    int32_t pair_launches; /* out: launches of two iterations that ran (m16_batch_solve: with time_kernels only, and
+                              those of one kind for each of several kinds of instances count as one) */
     double pair_ms;        /* out: their summed device time (time_kernels only) */
     int32_t pair_zc;       /* out (single solve): planes per block of those launches */
     int32_t reserved;

@@ -523,11 +523,19 @@ struct BatchTables {
     float *partials = nullptr;
 };
 
+// events around the launches of two iterations of a run, and how many there were
+// (all kinds' launches of the same two iterations count as one)
+struct PairTimer {
+    cudaEvent_t begin = nullptr, end = nullptr;
+    int pairs = 0;
+};
+
 // Enqueues m iterations of the work items; `check` computes the residual sums
-// of the last one (the caller launches the check).  e: optional events around
-// each launch.  Returns the number of sweep launches of the tile kinds (their
-// buffers alternated that often) or -1 on a launch error.
-inline int enqueue_iterations(const BatchTables &T, int m, bool check, cudaStream_t st, int &launches)
+// of the last one (the caller launches the check).  Returns the number of sweep
+// launches of the tile kinds (their buffers alternated that often) or -1 on a
+// launch error.
+inline int enqueue_iterations(const BatchTables &T, int m, bool check, cudaStream_t st, int &launches,
+                              PairTimer *timer = nullptr)
 {
     cudaError_t e = cudaSuccess;
     auto keep = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
@@ -535,6 +543,8 @@ inline int enqueue_iterations(const BatchTables &T, int m, bool check, cudaStrea
     while (done < m) {
         const int k = (m - done) & 1 ? 1 : 2;
         const bool last = done + k == m;
+        const bool timed = timer && k == 2 && T.seg[kTileKinds] > T.seg[0];
+        if (timed && timer->pairs++ == 0) keep(cudaEventRecord(timer->begin, st));
         for (int kind = 0; kind < kTileKinds; ++kind) {
             const int items = T.seg[kind + 1] - T.seg[kind];
             if (items <= 0) continue;
@@ -544,6 +554,7 @@ inline int enqueue_iterations(const BatchTables &T, int m, bool check, cudaStrea
                                  (const unsigned *)T.state, T.partials, sweeps & 1));
             ++launches;
         }
+        if (timed && last) keep(cudaEventRecord(timer->end, st));
         done += k;
         ++sweeps;
     }

@@ -224,7 +224,7 @@ struct BatchRun {
 // Descriptors, uploads and the set-up kernels.  The uploads read the host
 // vectors of B until they have run.
 int batch_prepare(BatchRun &B, const m16_batch_volume *vols, int nvol, const m16_batch_instance *inst, int ninst,
-                  const m16_cut_params *params, char *ws, cudaStream_t st, int &launches)
+                  const m16_cut_params *params, char *ws, cudaStream_t st)
 {
     const BatchLayout &L = B.L;
     B.nvol = nvol;
@@ -451,10 +451,10 @@ int batch_configure(BatchRun &B, const m16_batch_volume *vols, int bps, const st
 // m iterations; with `check` the last one's residuals, else the buffers' state
 // is stored by a launch of its own where it changed.  False on a launch error.
 bool batch_run(const BatchTables &T, int ninst, const m16_cut_params &p, int m, bool check, cudaStream_t st,
-               int &launches)
+               int &launches, PairTimer *timer = nullptr)
 {
     if (m <= 0) return true;
-    const int sweeps = enqueue_iterations(T, m, check, st, launches);
+    const int sweeps = enqueue_iterations(T, m, check, st, launches, timer);
     if (sweeps < 0) return false;
     if (check) {
         ++launches;
@@ -491,7 +491,7 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
 {
     int launches = 0;
     {
-        const int r = batch_prepare(B, vols, nvol, inst, ninst, params, ws, st, launches);
+        const int r = batch_prepare(B, vols, nvol, inst, ninst, params, ws, st);
         if (r != M16_OK) return r;
     }
     const BatchTables &T = B.T;
@@ -563,21 +563,26 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
         M16_BT_TRY(cudaEventCreate(&t0));
         M16_BT_TRY(cudaEventCreate(&t1));
     }
-    // m iterations on st, timed when asked
+    // m iterations on st; timing: their launches of two iterations are timed;
+    // time_it (the tuner): all of them, into last_ms
     double pair_ms = 0.0, last_ms = 0.0;
     int pair_n = 0;
-    auto run = [&](int m, bool check, bool time_it) -> cudaError_t {
+    auto run = [&](int m, bool check, bool time_it = false) -> cudaError_t {
+        PairTimer timer;
+        timer.begin = t0;
+        timer.end = t1;
         cudaError_t e = time_it ? cudaEventRecord(t0, st) : cudaSuccess;
         if (e != cudaSuccess) return e;
-        if (!batch_run(T, ninst, *params, m, check, st, launches)) return cudaErrorLaunchFailure;
-        if (!time_it) return cudaGetLastError();
-        if ((e = cudaEventRecord(t1, st)) != cudaSuccess) return e;
+        if (!batch_run(T, ninst, *params, m, check, st, launches, timing ? &timer : nullptr))
+            return cudaErrorLaunchFailure;
+        if (!time_it && !timer.pairs) return cudaGetLastError();
+        if (time_it && (e = cudaEventRecord(t1, st)) != cudaSuccess) return e;
         if ((e = cudaEventSynchronize(t1)) != cudaSuccess) return e;
         float ms = 0.f;
         e = cudaEventElapsedTime(&ms, t0, t1);
         last_ms = ms;
-        pair_ms += ms;
-        pair_n += (m + 1) / 2;
+        pair_ms += timing ? ms : 0.f;
+        pair_n += timer.pairs;
         return e;
     };
     std::vector<unsigned> state(ninst);
@@ -592,7 +597,7 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
     // iteration 0 ends the first run of launches (it is a check)
     int it = 0;
     if (num_iter > 0) {
-        M16_BT_TRY(run(1, true, timing));
+        M16_BT_TRY(run(1, true));
         it = 1;
     }
     int tune_stage = tune ? 0 : -1;
@@ -614,7 +619,7 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
     M16_BT_TRY(read_state());
     while (it < num_iter && n_active > 0) {
         if (it - 1 + (int64_t)update >= num_iter) {   // no check left: the last iterations
-            M16_BT_TRY(run(num_iter - it, false, timing));
+            M16_BT_TRY(run(num_iter - it, false));
             it = num_iter;
             break;
         }
@@ -653,7 +658,7 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
             launches += graph_launches;
             it += per_graph * update;
         } else {
-            M16_BT_TRY(run(update, true, timing));
+            M16_BT_TRY(run(update, true));
             it += update;
         }
         M16_BT_TRY(read_state());
@@ -685,8 +690,8 @@ int batch_solve_cohort(BatchRun &B, const m16_batch_volume *vols, int nvol, cons
     if (stats) {
         stats->blocks_per_sm = bps;
         stats->launches += launches;
-        stats->pair_launches += timing ? pair_n : 0;
-        stats->pair_ms += timing ? pair_ms : 0.0;
+        stats->pair_launches += pair_n;
+        stats->pair_ms += pair_ms;
     }
     return M16_OK;
 }
@@ -793,7 +798,7 @@ static int batch_begin(const m16_batch_volume *vols, int32_t nvol, const m16_bat
     b->params = *params;
     cudaStream_t st = (cudaStream_t)stream;
     int launches = 0;
-    int r = batch_prepare(B, vols, nvol, inst, ninst, params, (char *)workspace, st, launches);
+    int r = batch_prepare(B, vols, nvol, inst, ninst, params, (char *)workspace, st);
     // the handle owns the host sources until the copies have run
     if (r == M16_OK) r = batch_configure(B, vols, kDefaultBps, std::vector<char>(ninst, 1), st);
     if (r == M16_OK) r = batch_setup_kernels(B, vols, st, launches);
