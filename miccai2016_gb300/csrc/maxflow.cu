@@ -688,11 +688,12 @@ namespace m16 {
 namespace {
 constexpr int64_t kStaticMaxVoxels = 262144;
 constexpr int kStaticMaxChecks = 4096;
-// 88 B per padded voxel of the tile sweeps (at most 294,912 of them,
-// tile_shape_ok), 8 B per block of theirs (at least 208 voxels each, or all of a
-// small volume), max partials, control and residual log, each region rounded up
-// to 256 B; the two sweeps take less than half of it
-constexpr size_t kStaticBytes = 25u << 20;   // 25 MiB >= 25,990,000 B needed at the limits
+// The largest workspace of the tile sweeps at the limits, of all shapes: 88 B per
+// padded voxel (at most 294,912 of them, tile_shape_ok), 8 B per block (a block of
+// a volume of few columns or planes writes as few as 52 voxels: 5041 blocks at 1 x
+// 65536 x 4), max partials, control and residual log, each region rounded up to 256
+// B: 25,874,176 B (2097 x 5 x 25).  The two sweeps take less than half of it.
+constexpr size_t kStaticBytes = 25u << 20;
 
 }  // namespace
 }  // namespace m16
