@@ -57,10 +57,14 @@ typedef struct m16_cut_params {
 } m16_cut_params;
 
 /* Workspace bytes of m16_maxflow_solve for a (d0, d1, d2) volume: about 88 per
- * voxel, for the tile sweeps (two iterations per pass over memory; 76 do with
- * constant eigenvalues).  m16_maxflow_workspace_bytes_min is the least the
- * solve accepts: about 36 per voxel, with which every iteration is a flow and
- * a label launch, as it is for volumes of more than 2^31 padded voxels. */
+ * voxel, for the tile sweeps (two iterations per pass over memory); 76 do with
+ * constant eigenvalues (m16_maxflow_workspace_bytes_const).
+ * m16_maxflow_workspace_bytes_min is the least the solve accepts: about 36 per
+ * voxel, with which every iteration is a flow and a label launch, as it is for
+ * volumes of more than 2^31 padded voxels, of rows of more than 2^29, of rows
+ * that padding would lengthen by more than an eighth, and for large volumes of
+ * few rows. */
+size_t m16_maxflow_workspace_bytes_const(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 size_t m16_maxflow_workspace_bytes_min(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params);
 

@@ -102,6 +102,8 @@ def _declare(L):
     L.m16_maxflow_workspace_bytes.argtypes = [_i32, _i32, _i32, ctypes.POINTER(CutParams)]
     L.m16_maxflow_workspace_bytes_min.restype = _sz
     L.m16_maxflow_workspace_bytes_min.argtypes = L.m16_maxflow_workspace_bytes.argtypes
+    L.m16_maxflow_workspace_bytes_const.restype = _sz
+    L.m16_maxflow_workspace_bytes_const.argtypes = L.m16_maxflow_workspace_bytes.argtypes
     L.m16_maxflow_solve.restype = ctypes.c_int
     L.m16_maxflow_solve.argtypes = [_vp, _vp, _vp, _vp, _vp, _f32, _vp, _vp, _vp, _i32, _i32, _i32,
                                     ctypes.POINTER(CutParams), _vp, ctypes.POINTER(_i32), _vp, _i32,

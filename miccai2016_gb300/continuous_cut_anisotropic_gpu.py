@@ -120,7 +120,8 @@ class CmfCutQAnisotropicGpu(TreePrintable):
         p = self.params
         cp = N.CutParams(float(p.cc), float(p.steps), float(p.error_bound), int(p.num_iter), int(p.update),
                          (ctypes.c_double * 3)(*scaling))
-        nbytes = L.m16_maxflow_workspace_bytes(shape[0], shape[1], shape[2], ctypes.byref(cp))
+        size = L.m16_maxflow_workspace_bytes if sqc is None else L.m16_maxflow_workspace_bytes_const
+        nbytes = size(shape[0], shape[1], shape[2], ctypes.byref(cp))
         if self._ws is None or self._ws.numel() < nbytes:
             self._ws = None
             try:

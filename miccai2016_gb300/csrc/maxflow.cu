@@ -278,11 +278,21 @@ extern "C" size_t m16_maxflow_workspace_bytes_min(int32_t d0, int32_t d1, int32_
     return mf_layout(d0, d1, d2, params->num_iter, params->update).total;
 }
 
-extern "C" size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
+static size_t maxflow_workspace(int d0, int d1, int d2, const m16_cut_params *params, bool field)
 {
     const size_t two_sweeps = m16_maxflow_workspace_bytes_min(d0, d1, d2, params);
     if (!two_sweeps || !tile_shape_ok(d0, d1, d2)) return two_sweeps;
-    return std::max(two_sweeps, mf_tile_layout(d0, d1, d2, params->num_iter, params->update, true).total);
+    return std::max(two_sweeps, mf_tile_layout(d0, d1, d2, params->num_iter, params->update, field).total);
+}
+
+extern "C" size_t m16_maxflow_workspace_bytes(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
+{
+    return maxflow_workspace(d0, d1, d2, params, true);
+}
+
+extern "C" size_t m16_maxflow_workspace_bytes_const(int32_t d0, int32_t d1, int32_t d2, const m16_cut_params *params)
+{
+    return maxflow_workspace(d0, d1, d2, params, false);
 }
 
 extern "C" int m16_maxflow_solve(const float *img, const float *quat3, const double *sqevals3,
