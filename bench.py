@@ -10,9 +10,9 @@ iterations (residual checked every 30).  One step = one solve.
   value  solves/s with the inputs resident in HBM (all ranks summed)
   e2e    solves/s through the drop-in CmfCutQAnisotropicGpu.execute() with
          pinned host inputs: H2D of the inputs and D2H of u inside every step
-  roofline  the flow sweep (the dominant kernel of an iteration: flow 44 B,
-         labels 40 B per voxel), its launch time measured with CUDA events on
-         the solve's stream in a second pass over the same solves
+  roofline  the launch of two iterations (72 B per voxel), its time measured
+         with CUDA events on the solve's stream in a second pass over the same
+         solves
 
 python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 Under torchrun every rank runs its own replica (the solves are independent).
@@ -525,7 +525,8 @@ def run_batched_grid():
            "iterations": {"min": int(iters.min()), "median": float(np.median(iters)), "max": int(iters.max())},
            "voxel_iterations_per_s": vox_it_b / batched_s, "plain_voxel_iterations_per_s": vox_it_p / plain_s,
            "speedup_voxel_iterations_per_s": (vox_it_b / batched_s) / (vox_it_p / plain_s),
-           "achieved_gbs_state": 60.0 * vox_it_b / batched_s / 1e9,   # 60 B of per-instance state per voxel-iteration
+           # 48 B of an instance's state per voxel and two iterations
+           "achieved_gbs_state": 24.0 * vox_it_b / batched_s / 1e9,
            "best_dice_fast": float(dice_b[best]), "best_weighting": grid[best][0], "best_decay": grid[best][1],
            "best_dice_largest_component": best_dice_true, "plain_best_dice_largest_component": plain_best_dice_true,
            "dice_largest_component_s": dice_largest_s,

@@ -115,7 +115,7 @@ typedef struct m16_solve_stats {
     int32_t u_launches;    /* out: label (U) kernel launches that ran (0 with the tile sweeps) */
     double p_ms;           /* out: summed device time of the P launches (time_kernels only) */
     double u_ms;           /* out: summed device time of the U launches (time_kernels only) */
-    int32_t path;          /* in: M16_PATH_* -- how an iteration is launched */
+    int32_t path;          /* in: M16_PATH_* -- how an iteration is launched (m16_batch_solve takes both and has one way) */
     int32_t flags;         /* in: M16_BATCH_* options of m16_batch_solve (0 elsewhere) */
     int32_t blocks_per_sm; /* out (m16_batch_solve): the sweeps' tile shape in use at the end: 16 is the
                               default chunk of planes per block, 8 twice and 32 half of it; in, with

@@ -370,7 +370,8 @@ def served_vs_plain(n_requests=96, rate=50.0, pool=8, seed=0, max_resident=None,
                 server_steps=int(info["steps"] - info0["steps"]),
                 server_gpu_busy=gpu_s / latency_summary(served)["span_s"],
                 server_voxel_iterations_per_gpu_s=vox_it / gpu_s if gpu_s > 0 else None,
-                server_gbs_at_84B_per_voxel_iteration=84.0 * vox_it / gpu_s / 1e9 if gpu_s > 0 else None)
+                # a launch of two iterations moves 72 bytes a voxel
+                server_gbs_at_36B_per_voxel_iteration=36.0 * vox_it / gpu_s / 1e9 if gpu_s > 0 else None)
 
 
 def _main(argv=None):
