@@ -27,9 +27,10 @@
 // so captured launches can be replayed.
 //
 // Measured on GB300: 16 grid points at 128^3, anisotropic and isotropic (32
-// instances), 358 -> 152 ms against groups of four interleaved instances in a
-// flow and a label launch per iteration; eight uneven volumes 39.6 -> 18.5 ms;
-// ten served requests 113 -> 51 ms.  Bound by HBM where the tiles fit the
+// instances), 358 -> 155 ms against groups of four interleaved instances in a
+// flow and a label launch per iteration; eight uneven volumes 39.6 -> 20.0 ms;
+// ten served requests 113 -> 52 ms; 16 single planes of 256^2 alone are slower
+// (120 iterations 2.60 -> 3.16 ms).  Bound by HBM where the tiles fit the
 // volume (48 bytes of state per voxel and two iterations), by the march's
 // instructions on the halo where they do not (128^3: 1.56 times the voxels).
 //
