@@ -194,12 +194,23 @@ inline size_t batch_bytes(const m16_batch_volume *vols, int nvol, const m16_batc
     return std::max(kPairBudget, batch_layout(vols, nvol, inst, 0, ninst, true).total);
 }
 
-// The least that m16_batch_solve runs in: every instance alone, compact
+// The least that m16_batch_solve runs in: every instance alone, compact.  Such
+// layouts differ in these fields only, so one of them is laid out.
 inline size_t batch_bytes_min(const m16_batch_volume *vols, int nvol, const m16_batch_instance *inst, int ninst)
 {
-    size_t least = 0;
-    for (int i = 0; i < ninst; ++i) least = std::max(least, batch_layout(vols, nvol, inst, i, i + 1, true).total);
-    return least;
+    size_t most = 0;
+    int which = 0;
+    for (int i = 0; i < ninst; ++i) {
+        const m16_batch_volume &V = vols[inst[i].volume];
+        const size_t n = (size_t)V.d0 * V.d1 * V.d2, items = compact_tiles(V.d0, V.d1, V.d2);
+        const size_t bytes = align_up(n * 16, 256) + kFields * align_up(n * 4, 256) +
+                             align_up(items * sizeof(int2), 256) + align_up(items * sizeof(float), 256);
+        if (bytes > most) {
+            most = bytes;
+            which = i;
+        }
+    }
+    return batch_layout(vols, nvol, inst, which, which + 1, true).total;
 }
 
 // A batch's descriptors on host and device and its work list
